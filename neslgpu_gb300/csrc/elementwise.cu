@@ -104,14 +104,48 @@ __host__ __device__ inline Affine48 power48(unsigned long long e) {
   }
   return r;
 }
-__global__ void k_rand(int *__restrict__ d, const int *__restrict__ s, long n,
-                       unsigned long long x0) {
-  const long stride = (long)gridDim.x * EBLOCK;
-  for (long i = (long)blockIdx.x * EBLOCK + threadIdx.x; i < n; i += stride) {
-    Affine48 f = power48((unsigned long long)i + 1);
-    unsigned long long x = (f.a * x0 + f.c) & 0xFFFFFFFFFFFFULL;
-    int r = (int)(x >> 17);
-    d[i] = r % __ldg(s + i);
+// Element i draws X_{i+1}.  A thread reaches its first element's state by
+// applying the maps of 2^k draws for the set bits of i+1 (a table the host
+// passes: at most 32 multiply-adds), its next elements by one more
+// multiply-add each (256 draws on) and its next group by the map of a whole
+// grid stride.  Composing the maps by binary powering in every element cost
+// about 900 instructions each: 16.8 M draws 490 -> 40 us (the floor of 8
+// B per draw is 20 us; the rest is the division by the bound).
+struct RandSteps {
+  unsigned long long x0;         // state before the first draw
+  Affine48 pow2[32];             // pow2[k]: 2^k draws
+  Affine48 stride;               // the draws of a grid stride
+};
+constexpr int RAND_BLOCK_LOG2 = 8;
+static_assert(EBLOCK == 1 << RAND_BLOCK_LOG2, "elements of a thread's group lie a power of two of draws apart");
+__device__ __forceinline__ unsigned long long draw48(const Affine48 &f, unsigned long long x) {
+  return (f.a * x + f.c) & 0xFFFFFFFFFFFFULL;
+}
+__global__ void __launch_bounds__(EBLOCK) k_rand(int *__restrict__ d, const int *__restrict__ s, long n,
+                                                 const __grid_constant__ RandSteps r) {
+  const long stride = (long)gridDim.x * EBLOCK * EUNROLL;
+  long b = (long)blockIdx.x * EBLOCK * EUNROLL + threadIdx.x;
+  if (b >= n) return;
+  unsigned long long x = r.x0;
+  const unsigned e = (unsigned)(b + 1);
+#pragma unroll 1
+  for (int k = 0; k < 32 && (e >> k) != 0u; k++)
+    if ((e >> k) & 1u) x = draw48(r.pow2[k], x);
+  for (; b < n; b += stride) {
+    int m[EUNROLL];
+#pragma unroll
+    for (int u = 0; u < EUNROLL; u++) {
+      const long i = b + (long)u * EBLOCK;
+      m[u] = i < n ? __ldcs(s + i) : 1;
+    }
+    unsigned long long y = x;
+#pragma unroll
+    for (int u = 0; u < EUNROLL; u++) {
+      const long i = b + (long)u * EBLOCK;
+      if (i < n) d[i] = (int)(y >> 17) % m[u];
+      y = draw48(r.pow2[RAND_BLOCK_LOG2], y);
+    }
+    x = draw48(r.stride, x);
   }
 }
 
@@ -249,7 +283,13 @@ GCVL_EXPORT void rnd_wuz(vec_p d, vec_p s, int len, vec_p scratch) {
   (void)scratch; ensure_init();
   if (len <= 0) return;
   State &S = st();
-  k_rand<<<ew_grid(len), EBLOCK, 0, S.stream>>>((int *)d, (const int *)s, len, S.rand48);
+  const int grid = ew_grid(len);
+  RandSteps r;
+  r.x0 = S.rand48;
+  r.pow2[0] = power48(1);
+  for (int k = 1; k < 32; k++) r.pow2[k] = compose48(r.pow2[k - 1], r.pow2[k - 1]);
+  r.stride = power48((unsigned long long)grid * EBLOCK * EUNROLL);
+  k_rand<<<grid, EBLOCK, 0, S.stream>>>((int *)d, (const int *)s, len, r);
   launch_check("rnd_wuz");
   Affine48 f = power48((unsigned long long)len);
   S.rand48 = (f.a * S.rand48 + f.c) & 0xFFFFFFFFFFFFULL;
