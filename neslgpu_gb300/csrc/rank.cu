@@ -6,19 +6,22 @@
 // segment.  Keys are made order-preserving unsigned integers exactly as the
 // serial CVL does: int keys flip the sign bit (up) or every other bit
 // (down), rank.c:94-99; double keys flip all bits of negatives and the sign
-// bit of the rest, and down ranks complement that, rank.c:258-280.  A
-// segmented rank is a stable sort by (segment, key): the key passes carry
-// each element's segment number, then further passes sort by it.
+// bit of the rest, and down ranks complement that, rank.c:258-280.  The
+// digit passes rank long segments as a stable sort by (segment, key): the
+// key passes carry each element's segment number, then further passes sort
+// by it.
 //
-// GPU design (onesweep style).  One prepare pass builds every pass's 256-bin
-// digit histogram at once with shared-memory atomics (and, for segmented
-// ranks, writes transformed keys, indices and segment numbers).  Then one
-// pass per 8-bit digit: each warp of a CTA loads its 32 x RK_ITEMS
-// consecutive keys and values into registers, ranks them stably with
-// ballots, the CTA learns how many earlier tiles' elements fall in each
-// digit by a per-digit decoupled look-back, reorders the tile in shared
-// memory and writes coalesced runs.  The first pass of an unsegmented rank
-// reads the caller's keys and transforms them itself.
+// GPU design.  Segments of at most LR_MAX elements, and whole vectors of at
+// most LR_CAP, are ranked by one CTA each (rank_local.cu).  Longer vectors,
+// and the compacted long segments of a segmented rank, are sorted onesweep
+// style.  One prepare pass builds every pass's 256-bin digit histogram at
+// once with shared-memory atomics (and compacts the long segments' keys,
+// indices and segment numbers).  Then one pass per 8-bit digit: each warp of
+// a CTA loads its 32 x ITEMS consecutive keys and values into registers,
+// ranks them stably by lane masks, the CTA learns how many earlier tiles'
+// elements fall in each digit by a per-digit decoupled look-back, reorders
+// the tile in shared memory and writes coalesced runs.  The first pass of an
+// unsegmented rank reads the caller's keys and transforms them itself.
 //
 // The result is the inverse of the sort permutation: rank[index] = position,
 // a scatter to random places.  Below RK_DIRECT_MAX elements the last pass
@@ -32,7 +35,9 @@
 // flag permutes) split their pairs by window with passes of their own (the
 // window split below) and share the window scatter.
 #include "gcvl.cuh"
+#include "rank.cuh"
 
+#include <algorithm>
 #include <type_traits>
 #include <utility>
 
@@ -45,7 +50,7 @@ namespace gcvl {
 #ifndef GCVL_RK_ITEMS
 #define GCVL_RK_ITEMS 20
 #endif
-constexpr int RK_BLOCK = 256, RK_ITEMS = GCVL_RK_ITEMS, RK_TILE = RK_BLOCK * RK_ITEMS;
+constexpr int RK_BLOCK = 256, RK_ITEMS_LARGE = GCVL_RK_ITEMS;
 constexpr int RK_WARPS = RK_BLOCK / 32;
 constexpr int RK_MAXPASS = 12;
 #ifndef GCVL_RK_LB
@@ -60,7 +65,16 @@ constexpr int RK_MAXPASS = 12;
 #ifndef GCVL_RK_MINB_NARROW
 #define GCVL_RK_MINB_NARROW 3
 #endif
+// Vectors of at most 2^20 elements take smaller tiles, so that more CTAs work
+// (int / double ranks: 2^20 keys in tiles of 20 items 95 / 176 us, 16 items
+// 79 / 150, 8 items 88 / 173; 2^18 keys 67 / 117, 59 / 102, 55 / 100; at 2^21
+// 20 items win again, 108 / 244 against 121 / 232).
+#ifndef GCVL_RK_ITEMS_SMALL
+#define GCVL_RK_ITEMS_SMALL 16
+#endif
+constexpr int RK_ITEMS_SMALL = GCVL_RK_ITEMS_SMALL, RK_SMALL_MAX = 1 << 20;
 constexpr int RK_LB = GCVL_RK_LB;  // predecessors read per look-back round trip
+static_assert(RK_ITEMS_SMALL != RK_ITEMS_LARGE, "the tile tells the two forms apart");
 constexpr int RK_DIRECT_MAX = 1 << 23;
 // 8 measured best at 2^28 (bck_puz / smp_puz): 4 items 2.87 / 2.94 ms,
 // 8 items 2.63 / 2.78, 16 items 3.01 / 2.78
@@ -82,65 +96,98 @@ __host__ __device__ inline int bit_length(unsigned x) {
   return b;
 }
 
-struct RankPrep {
-  const void *src;
-  int n, is_double, up, seg, write_arrays;
-  SegView sv;
-  void *key;           // uint32 or uint64 transformed keys
-  unsigned *idx;
-  unsigned *aux;       // segment numbers (segmented ranks)
-  unsigned *hist;      // [RK_MAXPASS][256]
-  int key_passes, seg_passes;
-};
+__device__ __forceinline__ int key_digit(unsigned long long k, int q) { return (int)((k >> (8 * q)) & 255); }
 
-__device__ __forceinline__ unsigned long long rk_key64(unsigned long long b, int up) {
-  unsigned long long k = (b >> 63) ? ~b : (b ^ (1ULL << 63));
-  return up ? k : ~k;
-}
-__device__ __forceinline__ unsigned rk_key32(unsigned x, int up) { return x ^ (up ? 0x80000000u : 0x7FFFFFFFu); }
-
-__device__ __forceinline__ void rank_prep_one(const RankPrep &p, unsigned *s_hist, long i, unsigned long long raw) {
-  unsigned long long k;
-  if (p.is_double) {
-    k = rk_key64(raw, p.up);
-    if (p.write_arrays) ((unsigned long long *)p.key)[i] = k;
-  } else {
-    const unsigned kk = rk_key32((unsigned)raw, p.up);
-    if (p.write_arrays) ((unsigned *)p.key)[i] = kk;
-    k = kk;
-  }
-  if (p.write_arrays) p.idx[i] = (unsigned)i;
-  for (int q = 0; q < p.key_passes; q++) atomicAdd(&s_hist[q * 256 + (int)((k >> (8 * q)) & 255)], 1u);
-  if (p.seg) {
-    const unsigned sg = (unsigned)seg_of(p.sv, (int)i);
-    p.aux[i] = sg;
-    for (int q = 0; q < p.seg_passes; q++)
-      atomicAdd(&s_hist[(p.key_passes + q) * 256 + ((sg >> (8 * q)) & 255)], 1u);
-  }
-}
-__device__ __forceinline__ unsigned long long rank_prep_load(const RankPrep &p, long i) {
-  return p.is_double ? __ldcs((const unsigned long long *)p.src + i) : (unsigned long long)__ldcs((const unsigned *)p.src + i);
-}
-
-__global__ void __launch_bounds__(RK_BLOCK) k_rank_prep(RankPrep p) {
-  __shared__ unsigned s_hist[RK_MAXPASS * 256];
-  const int passes = p.key_passes + p.seg_passes;
-  for (int i = threadIdx.x; i < passes * 256; i += RK_BLOCK) s_hist[i] = 0;
-  __syncthreads();
+// Every key pass's 256-bin digit histogram of the caller's keys, in one read
+// of them, and the cleared look-back words of all passes.
+template <class K>
+__global__ void __launch_bounds__(RK_BLOCK) k_rank_prep(const K *__restrict__ src, int n, int up,
+                                                        unsigned *__restrict__ hist, uint4 *__restrict__ state,
+                                                        long state_vecs) {
+  constexpr int P = sizeof(K);
+  __shared__ unsigned s_hist[P * 256];
+  for (int i = threadIdx.x; i < P * 256; i += RK_BLOCK) s_hist[i] = 0;
   const long stride = (long)gridDim.x * RK_BLOCK;
   long i = (long)blockIdx.x * RK_BLOCK + threadIdx.x;
-  // four independent loads in flight per thread
-  for (; i + 3 * stride < p.n; i += 4 * stride) {
-    unsigned long long r[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) r[u] = rank_prep_load(p, i + u * stride);
-#pragma unroll
-    for (int u = 0; u < 4; u++) rank_prep_one(p, s_hist, i + u * stride, r[u]);
-  }
-  for (; i < p.n; i += stride) rank_prep_one(p, s_hist, i, rank_prep_load(p, i));
+  for (long w = i; w < state_vecs; w += stride) state[w] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  for (int i = threadIdx.x; i < passes * 256; i += RK_BLOCK)
-    if (s_hist[i]) atomicAdd(&p.hist[i], s_hist[i]);
+  // four independent loads in flight per thread
+  for (; i < n; i += 4 * stride) {
+    K r[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i + u * stride < n) r[u] = rk_key(__ldcs(src + i + u * stride), up);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i + u * stride < n)
+#pragma unroll
+        for (int q = 0; q < P; q++) atomicAdd(&s_hist[q * 256 + key_digit(r[u], q)], 1u);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < P * 256; b += RK_BLOCK)
+    if (s_hist[b]) atomicAdd(&hist[b], s_hist[b]);
+}
+
+// The long segments of a segmented rank: their keys, indices and segment
+// numbers into the compacted vector, the digit histograms of the key and the
+// segment-number passes, and the cleared look-back words of the compacted
+// vector's tiles.  A tile of LR_T elements holds at most two pieces of long
+// segments: the rest of one that started earlier and the start of another.
+// Returns at once when there are none.
+template <class K>
+__global__ void __launch_bounds__(RK_BLOCK) k_rank_prep_long(const K *__restrict__ src, int n, int up, SegView sv,
+                                                             LongSegs ls, int seg_passes, K *__restrict__ key,
+                                                             unsigned *__restrict__ idx, unsigned *__restrict__ aux,
+                                                             unsigned *__restrict__ hist, unsigned *__restrict__ state,
+                                                             long state_words, int tile_elems) {
+  constexpr int P = sizeof(K);
+  __shared__ unsigned s_hist[RK_MAXPASS * 256];
+  __shared__ int s_num[2], s_from[2], s_to[2];
+  const long total = (long)(unsigned)*(volatile const unsigned long long *)ls.total;
+  if (total == 0) return;
+  const int tid = threadIdx.x, bins = (P + seg_passes) * 256;
+  for (int i = tid; i < bins; i += RK_BLOCK) s_hist[i] = 0;
+  const long words = (total + tile_elems - 1) / tile_elems * 256;
+  for (long w = (long)blockIdx.x * RK_BLOCK + tid; w < 3 * words; w += (long)gridDim.x * RK_BLOCK)
+    state[w / words * state_words + w % words] = 0;
+  const int tiles = (int)(((long)n + LR_T - 1) / LR_T);
+  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+    __syncthreads();
+    const int lo = t * LR_T, hi = (int)min((long)lo + LR_T, (long)n);
+    if (tid < 2) {
+      int num = -1, a = 0, b = 0;
+      if (tid == 0) {  // the segment that covers the tile's first element, if it started earlier
+        const int s = seg_of(sv, lo), o = __ldg(sv.off + s), e = __ldg(sv.off + s + 1);
+        if (o < lo && e - o > LR_MAX) { num = ls.of_tile[o / LR_T]; a = lo; b = min(e, hi); }
+      } else if ((num = ls.of_tile[t]) >= 0) {
+        a = ls.first[num];
+        b = hi;  // longer than a tile: at least up to the next tile
+      }
+      s_num[tid] = num; s_from[tid] = a; s_to[tid] = b;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < 2; p++) {
+      const int num = s_num[p];
+      if (num < 0) continue;
+      const int first = ls.first[num], base = ls.base[num];
+      for (int i = s_from[p] + tid; i < s_to[p]; i += RK_BLOCK) {
+        const K k = rk_key(__ldcs(src + i), up);
+        const int c = base + (i - first);
+        key[c] = k;
+        idx[c] = (unsigned)i;
+        aux[c] = (unsigned)num;
+#pragma unroll
+        for (int q = 0; q < P; q++) atomicAdd(&s_hist[q * 256 + key_digit(k, q)], 1u);
+      }
+      if (tid == 0)
+        for (int q = 0; q < seg_passes; q++)
+          atomicAdd(&s_hist[(P + q) * 256 + ((num >> (8 * q)) & 255)], (unsigned)(s_to[p] - s_from[p]));
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < bins; i += RK_BLOCK)
+    if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
 // d[idx[i]] = s[i] when the indices ascend (gate word zero): the stores of a
@@ -167,51 +214,26 @@ __global__ void __launch_bounds__(RK_BLOCK) k_sorted_scatter(V *__restrict__ d, 
   }
 }
 
-// hist[q][d] -> exclusive scan over d, in place (one CTA, 256 threads)
-__global__ void k_rank_digit_starts(unsigned *hist, int passes) {
-  __shared__ unsigned s[256];
-  for (int q = 0; q < passes; q++) {
-    unsigned v = hist[q * 256 + threadIdx.x];
-    s[threadIdx.x] = v;
-    __syncthreads();
-    for (int d = 1; d < 256; d <<= 1) {
-      unsigned o = threadIdx.x >= d ? s[threadIdx.x - d] : 0u;
-      __syncthreads();
-      s[threadIdx.x] += o;
-      __syncthreads();
-    }
-    hist[q * 256 + threadIdx.x] = s[threadIdx.x] - v;
-    __syncthreads();
-  }
-}
-
-// digit starts of a permutation of [0, n) split by index >> shift: every
-// window but the last is full
-__global__ void k_window_starts(unsigned *starts, int n, int shift) {
-  const long s = (long)threadIdx.x << shift;
-  starts[threadIdx.x] = (unsigned)(s < n ? s : n);
-}
-
 template <class K, class V> struct PassArgs {
   const K *kin; const V *vin; const unsigned *ain;
   K *kout; V *vout; unsigned *aout;
   const void *src; int up;            // IN_SRC: the caller's keys
-  int *rank; const int *segoff;       // OUT_RANK / OUT_WIN (segmented: rebase by the key)
+  int *rank; const int *segbase;      // OUT_RANK / OUT_WIN (segment passes: the segments' first places)
   unsigned *pidx, *ppos;              // OUT_WIN
-  const unsigned *starts;             // this pass's digit starts
+  const unsigned *hist;               // this pass's digit counts
   unsigned *state;                    // [tiles][256] look-back words
-  const unsigned *wstarts;            // OUT_WIN: first slot of every output window
+  unsigned *clear;                    // another pass's look-back words, cleared for a later one
   unsigned *wstate;                   // OUT_WIN: [tiles][256] look-back words of the window counts
   int wshift;                         // OUT_WIN: window of v = v >> wshift
   unsigned *counter;
-  const unsigned *gate;               // non-null: the pass runs only if *gate is non-zero
+  const unsigned long long *total;    // DYN: the vector's length is the low word
   int n, shift;
   unsigned *status;
   int spin_limit;
 };
 
-template <class K, class V, bool AUX> constexpr size_t pass_smem() {
-  return (size_t)RK_TILE * (sizeof(K) + sizeof(V) + (AUX ? 4 : 0)) + RK_WARPS * 256 * 2 + 256 * 4 + 256 * 8;
+template <class K, class V, bool AUX, int ITEMS> constexpr size_t pass_smem() {
+  return (size_t)RK_BLOCK * ITEMS * (sizeof(K) + sizeof(V) + (AUX ? 4 : 0)) + RK_WARPS * 256 * 4 + 256 * 4 + 256 * 8;
 }
 
 // Publish this tile's count of one bin (digit or window), then look back for
@@ -259,12 +281,11 @@ __device__ __forceinline__ unsigned bin_lookback(unsigned *state, int tile, int 
   return prefix;
 }
 
-// Equal digits keep their order (the ballots below rank each warp's
-// elements in element order).
+// Equal digits keep their order (each warp ranks its elements in element order).
 template <class K, bool AUX> constexpr int rk_minb() { return sizeof(K) == 4 && !AUX ? GCVL_RK_MINB_NARROW : GCVL_RK_MINB; }
-template <class K, class V, bool AUX, int IN, int OUT>
-__global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(PassArgs<K, V> a) {
-  typedef unsigned short CntT;  // per-warp digit counts (at most 32 * RK_ITEMS)
+template <class K, class V, bool AUX, int IN, int OUT, int ITEMS>
+__device__ __forceinline__ void radix_tile(const PassArgs<K, V> &a, const int n, const int tile) {
+  constexpr int RK_ITEMS = ITEMS, RK_TILE = RK_BLOCK * ITEMS;
   // 32-bit keys and values leave the reorder as one 8-byte pair
   constexpr bool PAIR = sizeof(K) == 4 && sizeof(V) == 4 && OUT == OUT_ARRAYS;
   extern __shared__ __align__(16) unsigned char rk_smem[];
@@ -275,18 +296,16 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
   uint2 *s_pair = (uint2 *)s_kout;                         // PAIR: [RK_TILE] (key, value)
   unsigned *s_aout = (unsigned *)(s_vout + RK_TILE);
   unsigned *s_loc = s_aout + (AUX ? RK_TILE : 0);          // [256] tile offset per digit
-  CntT *s_cnt = (CntT *)(s_loc + 256);                      // [RK_WARPS][256]
-  __shared__ unsigned s_tile;
-  __shared__ unsigned s_ws[RK_WARPS];
+  unsigned *s_cnt = s_loc + 256;                           // [RK_WARPS][256]
+  __shared__ unsigned s_ws[RK_WARPS], s_hs[RK_WARPS];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (a.gate && *(const volatile unsigned *)a.gate == 0) return;  // the same answer for every CTA
-  if (tid == 0) s_tile = atomicAdd(a.counter, 1u);
   for (int i = tid; i < RK_WARPS * 256; i += RK_BLOCK) s_cnt[i] = 0;
+  for (int i = tid; i < RK_ITEMS / 4 * RK_WARPS * 256 / 4; i += RK_BLOCK)
+    ((uint4 *)s_kout)[i] = make_uint4(0, 0, 0, 0);  // the lane masks
   __syncthreads();
-  const int tile = (int)s_tile;
   const long base = (long)tile * RK_TILE;
-  const int valid = (int)min((long)RK_TILE, (long)a.n - base);
+  const int valid = (int)min((long)RK_TILE, (long)n - base);
 
   // each warp's 32 * RK_ITEMS consecutive elements straight into registers
   // (element wbase + 32c + lane in item c: coalesced, every load in flight)
@@ -297,15 +316,13 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
 #pragma unroll
   for (int c = 0; c < RK_ITEMS; c++) {
     const int e = wbase + c * 32 + lane;
-    kr[c] = 0;
+    // past the vector's end: the largest digit, ranked behind the tile's own
+    kr[c] = ~(K)0;
     vr[c] = 0;
     if (AUX) ar[c] = 0;
     if (e < valid) {
       if constexpr (IN == IN_SRC) {
-        if constexpr (sizeof(K) == 8)
-          kr[c] = (K)rk_key64(__ldcs((const unsigned long long *)a.src + base + e), a.up);
-        else
-          kr[c] = (K)rk_key32(__ldcs((const unsigned *)a.src + base + e), a.up);
+        kr[c] = rk_key(__ldcs((const K *)a.src + base + e), a.up);
         vr[c] = (V)(base + e);
       } else {
         kr[c] = __ldcs(a.kin + base + e);
@@ -315,55 +332,86 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
     }
   }
 
-  // rank within each warp's 512 elements: (rank << 8) | digit
-  CntT *cnt = s_cnt + warp * 256;
+  // Rank within each warp's elements: (rank << 8) | digit.  An item's peers
+  // (the lanes with its digit) come from a lane mask per digit in shared
+  // memory, where the tile is reordered later: every lane sets its bit, reads
+  // the mask back, and the first peer counts for all and clears it; G items
+  // at a time with masks of their own, so that their accesses are in flight
+  // together.  Eight ballots an item (four ALU instructions a bit) kept the
+  // ALU busy and the shared-memory pipe idle: a pass over 2^26 keys 406 us,
+  // now 366 us with the shared-memory pipe 77 % busy.  Ballots for one, two
+  // or three of every five items changed nothing or lost.
+  unsigned *cnt = s_cnt + warp * 256;
   const unsigned lt = (1u << lane) - 1u;
+  constexpr int G = RK_ITEMS / 4;
+  unsigned *mask = (unsigned *)s_kout + warp * 256;  // [G][RK_WARPS][256]
+  static_assert((size_t)G * RK_WARPS * 256 * 4 <= (size_t)RK_TILE * (sizeof(K) + sizeof(V)) && RK_ITEMS % G == 0,
+                "the masks fit where the tile is reordered");
   unsigned wr[RK_ITEMS];
 #pragma unroll
-  for (int c = 0; c < RK_ITEMS; c++) {
-    const int e = wbase + c * 32 + lane;
-    const int d = e < valid ? (int)((kr[c] >> a.shift) & 255) : -1;
-    unsigned r = 0;
-    const unsigned peers = warp_match8(d);
-    if (d >= 0) r = cnt[d] + __popc(peers & lt);
+  for (int c0 = 0; c0 < RK_ITEMS; c0 += G) {
+    unsigned m[G];
+#pragma unroll
+    for (int u = 0; u < G; u++)
+      atomicOr(mask + u * RK_WARPS * 256 + ((unsigned)(kr[c0 + u] >> a.shift) & 255u), 1u << lane);
     __syncwarp();
-    if (d >= 0 && (peers & lt) == 0) cnt[d] = (CntT)(cnt[d] + __popc(peers));
+#pragma unroll
+    for (int u = 0; u < G; u++) m[u] = mask[u * RK_WARPS * 256 + ((unsigned)(kr[c0 + u] >> a.shift) & 255u)];
     __syncwarp();
-    wr[c] = d >= 0 ? (r << 8) | (unsigned)d : 0xFFFFFFFFu;
+#pragma unroll
+    for (int u = 0; u < G; u++) {
+      const unsigned d = (unsigned)(kr[c0 + u] >> a.shift) & 255u;
+      unsigned r = 0;
+      if ((m[u] & lt) == 0) {
+        r = atomicAdd(cnt + d, (unsigned)__popc(m[u]));
+        mask[u * RK_WARPS * 256 + d] = 0;
+      }
+      wr[c0 + u] = r;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < G; u++) {
+      const unsigned d = (unsigned)(kr[c0 + u] >> a.shift) & 255u;
+      wr[c0 + u] = ((shfl_idx(wr[c0 + u], __ffs(m[u]) - 1) + __popc(m[u] & lt)) << 8) | d;
+    }
   }
   __syncthreads();
 
   // per digit: tile count, per-warp exclusive offsets
   const int dd = tid;  // RK_BLOCK == 256 digits
+  if (OUT == OUT_ARRAYS && a.clear) a.clear[(long)tile * 256 + dd] = 0;
   unsigned tot = 0;
 #pragma unroll
   for (int w = 0; w < RK_WARPS; w++) {
     unsigned c = s_cnt[w * 256 + dd];
-    s_cnt[w * 256 + dd] = (CntT)tot;
+    s_cnt[w * 256 + dd] = tot;
     tot += c;
   }
   const unsigned prefix = bin_lookback(a.state, tile, dd, tot, a.status, a.spin_limit);
-  // exclusive scan of tile counts over the digits -> tile offsets
+  // exclusive scans over the digits of the tile's counts -> tile offsets,
+  // and of the vector's counts -> digit starts
   {
-    unsigned incl = tot;
+    const unsigned all = __ldg(a.hist + dd);
+    unsigned incl = tot, hincl = all;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      unsigned x = shfl_up(incl, o);
-      if (lane >= o) incl += x;
+      const unsigned x = shfl_up(incl, o), y = shfl_up(hincl, o);
+      if (lane >= o) { incl += x; hincl += y; }
     }
-    if (lane == 31) s_ws[warp] = incl;
+    if (lane == 31) { s_ws[warp] = incl; s_hs[warp] = hincl; }
     __syncthreads();
-    unsigned wp = 0;
+    unsigned wp = 0, hp = 0;
 #pragma unroll
-    for (int w = 0; w < RK_WARPS; w++) if (w < warp) wp += s_ws[w];
+    for (int w = 0; w < RK_WARPS; w++)
+      if (w < warp) { wp += s_ws[w]; hp += s_hs[w]; }
     const unsigned loc = wp + incl - tot;
     s_loc[dd] = loc;
-    s_gb[dd] = (long long)__ldg(a.starts + dd) + (long long)prefix - (long long)loc;
+    s_gb[dd] = (long long)(hp + hincl - all) + (long long)prefix - (long long)loc;
     // each warp's counter of this digit becomes the digit's slot in the
     // reordered tile for that warp (one shared-memory lookup per element
-    // below instead of two; below 4096, so it fits the 16-bit counter)
+    // below instead of two)
 #pragma unroll
-    for (int w = 0; w < RK_WARPS; w++) s_cnt[w * 256 + dd] = (CntT)(s_cnt[w * 256 + dd] + loc);
+    for (int w = 0; w < RK_WARPS; w++) s_cnt[w * 256 + dd] += loc;
   }
   __syncthreads();
   if constexpr (OUT == OUT_WIN) {
@@ -375,22 +423,21 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
     unsigned pos[RK_ITEMS];
 #pragma unroll
     for (int c = 0; c < RK_ITEMS; c++) {
-      const unsigned x = wr[c];
+      const unsigned x = wr[c], d = x & 255u;
       pos[c] = 0;
-      if (x != 0xFFFFFFFFu) {
-        const int d = (int)(x & 255u);
+      if (wbase + c * 32 + lane < valid) {
         long long g = s_gb[d] + s_cnt[warp * 256 + d] + (x >> 8);
-        if (a.segoff) g -= __ldg(a.segoff + (int)kr[c]);
+        if (a.segbase) g -= __ldg(a.segbase + (int)kr[c]);
         pos[c] = (unsigned)g;
       }
     }
     __syncthreads();  // s_cnt, s_loc and s_gb are free
-    unsigned *s_wc = (unsigned *)s_cnt;  // [256] window counts
+    unsigned *s_wc = s_cnt;  // [256] window counts
     s_wc[tid] = 0;
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < RK_ITEMS; c++) {
-      if (wr[c] != 0xFFFFFFFFu) {
+      if (wbase + c * 32 + lane < valid) {
         const unsigned w = (unsigned)vr[c] >> a.wshift;
         wr[c] = (atomicAdd(s_wc + w, 1u) << 8) | w;
       }
@@ -412,14 +459,15 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
       for (int w = 0; w < RK_WARPS; w++) if (w < warp) wp += s_ws[w];
       const unsigned wloc = wp + incl - wtot;
       s_loc[tid] = wloc;
-      s_gb[tid] = (long long)__ldg(a.wstarts + tid) + (long long)wprefix - (long long)wloc;
+      // distinct indices: window w's pairs have room from its first index on
+      s_gb[tid] = ((long long)tid << a.wshift) + (long long)wprefix - (long long)wloc;
     }
     __syncthreads();
     uint2 *s_vp = (uint2 *)s_kout;  // (v, position) by window slot: one 8-byte store
 #pragma unroll
     for (int c = 0; c < RK_ITEMS; c++) {
       const unsigned x = wr[c];
-      if (x != 0xFFFFFFFFu) s_vp[s_loc[x & 255u] + (x >> 8)] = make_uint2((unsigned)vr[c], pos[c]);
+      if (wbase + c * 32 + lane < valid) s_vp[s_loc[x & 255u] + (x >> 8)] = make_uint2((unsigned)vr[c], pos[c]);
     }
     __syncthreads();
 #pragma unroll 4
@@ -431,21 +479,18 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
     }
     return;
   }
-  // reorder the tile in shared memory
+  // reorder the tile in shared memory (what lies past the vector's end lands
+  // past the tile's own elements)
 #pragma unroll
   for (int c = 0; c < RK_ITEMS; c++) {
-    const unsigned x = wr[c];
-    if (x != 0xFFFFFFFFu) {
-      const int d = (int)(x & 255u);
-      const unsigned lp = s_cnt[warp * 256 + d] + (x >> 8);
-      if constexpr (PAIR) {
-        s_pair[lp] = make_uint2((unsigned)kr[c], (unsigned)vr[c]);
-      } else {
-        s_kout[lp] = kr[c];
-        s_vout[lp] = vr[c];
-      }
-      if (AUX) s_aout[lp] = ar[c];
+    const unsigned lp = s_cnt[warp * 256 + (wr[c] & 255u)] + (wr[c] >> 8);
+    if constexpr (PAIR) {
+      s_pair[lp] = make_uint2((unsigned)kr[c], (unsigned)vr[c]);
+    } else {
+      s_kout[lp] = kr[c];
+      s_vout[lp] = vr[c];
     }
+    if (AUX) s_aout[lp] = ar[c];
   }
   __syncthreads();
   // coalesced runs out
@@ -469,9 +514,35 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
       if (AUX) a.aout[g] = s_aout[e];
     } else {  // OUT_RANK
       int r = (int)g;
-      if (a.segoff) r -= __ldg(a.segoff + (int)k);
+      if (a.segbase) r -= __ldg(a.segbase + (int)k);
       a.rank[(unsigned)vv] = r;
     }
+  }
+}
+
+// One tile per CTA, taken in ticket order.  DYN: the vector's length is only
+// known on the device (long segments, usually none), so a resident grid
+// takes tiles until there are no more and costs one empty launch otherwise
+// (a grid for the longest possible vector: 5-7 us of CTAs that return).
+template <class K, class V, bool AUX, int IN, int OUT, int ITEMS, bool DYN>
+__global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(PassArgs<K, V> a) {
+  __shared__ unsigned s_tile;
+  if constexpr (DYN) {
+    const long n = (long)(unsigned)*(volatile const unsigned long long *)a.total;
+    const int tiles = (int)((n + RK_BLOCK * ITEMS - 1) / (RK_BLOCK * ITEMS));
+    if ((int)blockIdx.x >= tiles) return;
+    while (true) {
+      if (threadIdx.x == 0) s_tile = atomicAdd(a.counter, 1u);
+      __syncthreads();
+      const int tile = (int)s_tile;
+      if (tile >= tiles) return;
+      radix_tile<K, V, AUX, IN, OUT, ITEMS>(a, (int)n, tile);
+      __syncthreads();
+    }
+  } else {
+    if (threadIdx.x == 0) s_tile = atomicAdd(a.counter, 1u);
+    __syncthreads();
+    radix_tile<K, V, AUX, IN, OUT, ITEMS>(a, a.n, (int)s_tile);
   }
 }
 
@@ -721,20 +792,28 @@ __global__ void __launch_bounds__(RK_BLOCK) k_gather_gated(V *__restrict__ d, co
   }
 }
 
-template <class K, class V, bool AUX, int IN, int OUT>
-void launch_pass(const PassArgs<K, V> &a, int tiles) {
-  constexpr size_t sm = pass_smem<K, V, AUX>();
+template <class K, class V, bool AUX, int IN, int OUT, int ITEMS, bool DYN>
+void launch_pass_items(const PassArgs<K, V> &a) {
+  constexpr size_t sm = pass_smem<K, V, AUX, ITEMS>();
   static bool attr = false;
   if (!attr) {
-    GCVL_CK(cudaFuncSetAttribute(k_radix_pass<K, V, AUX, IN, OUT>,
+    GCVL_CK(cudaFuncSetAttribute(k_radix_pass<K, V, AUX, IN, OUT, ITEMS, DYN>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     attr = true;
   }
-  k_radix_pass<K, V, AUX, IN, OUT><<<tiles, RK_BLOCK, sm, stream()>>>(a);
+  int grid = ceil_div(a.n, RK_BLOCK * ITEMS);
+  if (DYN) grid = std::min(grid, st().sm_count * rk_minb<K, AUX>());
+  k_radix_pass<K, V, AUX, IN, OUT, ITEMS, DYN><<<grid, RK_BLOCK, sm, stream()>>>(a);
   launch_check("k_radix_pass");
 }
+inline bool rk_small(long n) { return n <= RK_SMALL_MAX; }
+inline int rk_tile(long n) { return RK_BLOCK * (rk_small(n) ? RK_ITEMS_SMALL : RK_ITEMS_LARGE); }
+template <class K, class V, bool AUX, int IN, int OUT, bool DYN> void launch_pass(const PassArgs<K, V> &a) {
+  if (!rk_small(a.n)) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_LARGE, DYN>(a);
+  else if constexpr (OUT != OUT_WIN) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_SMALL, DYN>(a);
+}
+static_assert(RK_SMALL_MAX <= RK_DIRECT_MAX, "windows only for large tiles");
 
-inline int rk_tiles(long n) { return (int)((n + RK_TILE - 1) / RK_TILE); }
 inline int sc_blocks(long n) { return (int)((n + RK_BLOCK * SC_ITEMS - 1) / (RK_BLOCK * SC_ITEMS)); }
 // grid of the sorted-index scatter: grid-stride over at most 16 CTAs per
 // SM, so that when its gate says "not this time" it costs a few
@@ -744,7 +823,7 @@ inline int sc_grid(long n) {
   const long cap = (long)st().sm_count * 16;
   return (int)(need < cap ? (need < 1 ? 1 : need) : cap);
 }
-inline size_t rk_state_bytes(long n) { return (size_t)rk_tiles(n) * 256 * 4; }
+inline size_t rk_state_bytes(long n) { return (size_t)ceil_div(n, rk_tile(n)) * 256 * 4; }
 inline int ws_tiles(long n) { return (int)((n + WS_TILE - 1) / WS_TILE); }  // tiles of the window split
 // top-8-bit windows of [0, n)
 inline int window_shift(int n) { int b = bit_length((unsigned)(n > 1 ? n - 1 : 1)); return b > 8 ? b - 8 : 0; }
@@ -910,27 +989,70 @@ template void scatter_partitioned<unsigned long long>(unsigned long long *, cons
                                                       const int *, int, int, vec_p);
 
 // ------------------------------------------------------------- rank ---
+// rank[index] = position from the (index, position) pairs of the last pass,
+// grouped by window of the index: window w's pairs lie from slot w << wshift
+// on, as many as the last pass counted (all the window's indices when the
+// vector was ranked whole).  One CTA per 2048 slots, as k_window_scatter;
+// DYN (long segments, usually none): a resident grid.
+template <bool DYN>
+__global__ void __launch_bounds__(RK_BLOCK) k_rank_scatter(int *__restrict__ rank, const unsigned *__restrict__ pidx,
+                                                           const unsigned *__restrict__ ppos, int n, int wshift,
+                                                           const unsigned long long *total,
+                                                           const unsigned *__restrict__ wstate, int tile_elems) {
+  const unsigned *counts = nullptr;  // the last tile's inclusive window counts
+  if constexpr (DYN) {
+    const long t = (long)(unsigned)*(volatile const unsigned long long *)total;
+    if (t == 0) return;
+    counts = wstate + (t - 1) / tile_elems * 256;
+  }
+  for (long b = blockIdx.x; b * (RK_BLOCK * SC_ITEMS) < n; b += gridDim.x) {
+    const long i0 = b * (RK_BLOCK * SC_ITEMS) + threadIdx.x;
+    unsigned k[SC_ITEMS], v[SC_ITEMS];
+    bool ok[SC_ITEMS];
+#pragma unroll
+    for (int u = 0; u < SC_ITEMS; u++) {
+      const long i = i0 + (long)u * RK_BLOCK;
+      ok[u] = i < n;
+      if (DYN && ok[u]) ok[u] = (i & ((1L << wshift) - 1)) < (long)(__ldg(counts + (i >> wshift)) & ~RK_INC);
+      if (ok[u]) { k[u] = __ldcs(pidx + i); v[u] = __ldcs(ppos + i); }
+    }
+#pragma unroll
+    for (int u = 0; u < SC_ITEMS; u++)
+      if (ok[u]) rank[k[u]] = (int)v[u];
+    if (!DYN) return;
+  }
+}
+
+// Scratch of the digit passes.  Whole vectors: pairs twice, digit counts,
+// look-back words three times over (a pass's own, those it clears for the
+// one after the next, and those in between; the last pass takes two).
+// Segmented: the same for the long segments, with their numbers and tables.
 struct RankLayout {
-  size_t key_a, key_b, idx_a, idx_b, aux_a, aux_b, hist, state, wstate, counter, total;
+  size_t hist, counter, lsum, state, key_a, key_b, idx_a, idx_b, aux_a, aux_b, first, base, of_tile, total;
 };
 inline RankLayout rank_layout(int n, int is_double, int seg) {
   RankLayout L;
   size_t ks = is_double ? 8 : 4;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += align_up(bytes, 256); return at; };
+  L.hist = take(RK_MAXPASS * 256 * 4);  // these three are cleared together
+  L.counter = take(RK_MAXPASS * 4);
+  L.lsum = take(8);
+  L.state = take(rk_state_bytes(n) * 3);
   L.key_a = take((size_t)n * ks);
   L.key_b = take((size_t)n * ks);
   L.idx_a = take((size_t)n * 4);
   L.idx_b = take((size_t)n * 4);
   L.aux_a = take(seg ? (size_t)n * 4 : 0);
   L.aux_b = take(seg ? (size_t)n * 4 : 0);
-  L.hist = take((RK_MAXPASS + 1) * 256 * 4);  // every pass's digit starts, then the window starts
-  L.counter = take((RK_MAXPASS + 1) * 4);
-  L.state = take(rk_state_bytes(n));
-  L.wstate = take(n > RK_DIRECT_MAX ? rk_state_bytes(n) : 0);  // the last pass's window look-back
+  L.first = take(seg ? ((size_t)n / LR_MAX + 1) * 4 : 0);
+  L.base = take(seg ? ((size_t)n / LR_MAX + 1) * 4 : 0);
+  L.of_tile = take(seg ? (size_t)lr_tiles(n) * 4 : 0);
   L.total = o + 256;  // room to align the base
   return L;
 }
+// one CTA ranks the whole vector: at most LR_CAP elements in at most LR_T segments
+inline bool rank_whole(int n, int m) { return n <= LR_CAP && (m <= LR_T || n <= LR_T); }
 int rank_units(int n, int is_double, int seg) {
   if (n <= 0) return 0;
   return (int)((rank_layout(n, is_double, seg).total + 7) / 8);
@@ -942,106 +1064,106 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
   State &S = st();
   if (n <= 0) return;
   const bool seg = sd != nullptr && m > 1;
-  RankLayout L = rank_layout(n, is_double, seg);
+  const SegView sv = seg ? seg_view(sd, n, m) : SegView{nullptr, nullptr, nullptr, nullptr, n, 1};
+  if (rank_whole(n, m)) {
+    rank_local<K>(s, (int *)d, sv, n, up, true, LongSegs{});
+    return;
+  }
+  const RankLayout L = rank_layout(n, is_double, seg);
   char *raw = (char *)scratch_or_work(scratch, L.total);
   if (!raw) return;
   char *mem = (char *)align_up((size_t)raw, 256);
-  const int key_passes = is_double ? 8 : 4;
-  int seg_passes = 0;
-  if (seg) seg_passes = (bit_length((unsigned)(m - 1)) + 7) / 8;
-  if (seg && seg_passes == 0) seg_passes = 1;
-  const int passes = key_passes + seg_passes;
-  const int tiles = rk_tiles(n);
-  const bool direct = n <= RK_DIRECT_MAX;
-  unsigned *hist = (unsigned *)(mem + L.hist);
-  unsigned *counters = (unsigned *)(mem + L.counter);
-  unsigned *state = (unsigned *)(mem + L.state);
-  GCVL_CK(cudaMemsetAsync(hist, 0, RK_MAXPASS * 256 * 4, S.stream));
-  GCVL_CK(cudaMemsetAsync(counters, 0, (RK_MAXPASS + 1) * 4, S.stream));
+  unsigned *hist = (unsigned *)(mem + L.hist), *counters = (unsigned *)(mem + L.counter);
+  const size_t state_bytes = rk_state_bytes(n);
+  unsigned *state[3];
+  for (int b = 0; b < 3; b++) state[b] = (unsigned *)(mem + L.state + b * state_bytes);
+  if (!GCVL_CK(cudaMemsetAsync(mem + L.hist, 0, L.state - L.hist, S.stream))) return;
 
-  // histograms of every pass (and, segmented, the staged keys)
-  RankPrep p;
-  p.src = s; p.n = n; p.is_double = is_double; p.up = up; p.seg = seg ? 1 : 0;
-  p.write_arrays = seg ? 1 : 0;
-  p.sv = seg ? seg_view(sd, n, m) : SegView{nullptr, nullptr, nullptr, nullptr, n, 1};
-  p.key = mem + L.key_a; p.idx = (unsigned *)(mem + L.idx_a);
-  p.aux = seg ? (unsigned *)(mem + L.aux_a) : nullptr;
-  p.hist = hist; p.key_passes = key_passes; p.seg_passes = seg_passes;
-  int pg = S.sm_count * 8;
-  long need = ((long)n + RK_BLOCK - 1) / RK_BLOCK;
-  if (pg > need) pg = (int)need;
-  k_rank_prep<<<pg, RK_BLOCK, 0, S.stream>>>(p);
-  launch_check("k_rank_prep");
-  k_rank_digit_starts<<<1, 256, 0, S.stream>>>(hist, passes);
-  launch_check("k_rank_digit_starts");
-
-  // ping-pong buffers
   char *kA = mem + L.key_a, *kB = mem + L.key_b;
   unsigned *iA = (unsigned *)(mem + L.idx_a), *iB = (unsigned *)(mem + L.idx_b);
-  unsigned *aA = seg ? (unsigned *)(mem + L.aux_a) : nullptr, *aB = seg ? (unsigned *)(mem + L.aux_b) : nullptr;
-  const int *segoff = seg ? seg_view(sd, n, m).off : nullptr;
-  // last pass output when the ranks go through the window partition: the
-  // pair arrays take the buffers the last pass does not read, grouped by
-  // the window of the index (256 windows of the rank vector)
-  unsigned *pidx = nullptr, *ppos = nullptr;
-  const int wshift = window_shift(n);
-  unsigned *wst = hist + RK_MAXPASS * 256;
-  unsigned *wstate = (unsigned *)(mem + L.wstate);
-  if (!direct) {
-    k_window_starts<<<1, 256, 0, S.stream>>>(wst, n, wshift);
-    launch_check("k_window_starts");
-    GCVL_CK(cudaMemsetAsync(wstate, 0, rk_state_bytes(n), S.stream));
+  unsigned *aA = (unsigned *)(mem + L.aux_a), *aB = (unsigned *)(mem + L.aux_b);
+  const int key_passes = (int)sizeof(K);
+  int seg_passes = 0;
+  const unsigned long long *total = nullptr;
+  const int *segbase = nullptr;
+  if (seg) {
+    LongSegs ls;
+    ls.total = (unsigned long long *)(mem + L.lsum);
+    ls.first = (int *)(mem + L.first);
+    ls.base = (int *)(mem + L.base);
+    ls.of_tile = (int *)(mem + L.of_tile);
+    rank_local<K>(s, (int *)d, sv, n, up, false, ls);
+    if (n <= LR_MAX) return;  // no segment can be longer
+    // the long segments, if there are any: the kernels below return at once otherwise
+    total = ls.total;
+    segbase = ls.base;
+    seg_passes = std::max(1, (bit_length((unsigned)(n / (LR_MAX + 1) - 1)) + 7) / 8);
+    const int pg = std::min(S.sm_count * 8, lr_tiles(n));
+    k_rank_prep_long<K><<<pg, RK_BLOCK, 0, S.stream>>>((const K *)s, n, up, sv, ls, seg_passes, (K *)kA, iA, aA, hist,
+                                                       state[0], (long)(state_bytes / 4), rk_tile(n));
+    launch_check("k_rank_prep_long");
+  } else {
+    const int pg = std::min(S.sm_count * 8, ceil_div(n, (long)RK_BLOCK));
+    k_rank_prep<K><<<pg, RK_BLOCK, 0, S.stream>>>((const K *)s, n, up, hist, (uint4 *)state[0],
+                                                  (long)(3 * state_bytes / 16));
+    launch_check("k_rank_prep");
   }
+
+  const int passes = key_passes + seg_passes;
+  const bool direct = n <= RK_DIRECT_MAX;
+  const int wshift = window_shift(n);
+  unsigned *pidx = nullptr, *ppos = nullptr, *wstate = nullptr;
   for (int q = 0; q < passes; q++) {
-    GCVL_CK(cudaMemsetAsync(state, 0, rk_state_bytes(n), S.stream));
     const bool final = (q == passes - 1);
-    const bool keypass = q < key_passes;
-    if (final) { pidx = iB; ppos = (unsigned *)kB; }
-    if (keypass) {
+    if (final) {  // the pairs by window take the buffers the last pass does not read
+      pidx = iB;
+      ppos = (unsigned *)kB;
+      wstate = state[(q + 1) % 3];
+    }
+    auto common = [&](auto &a) {
+      a.vin = iA;
+      a.vout = iB;
+      a.rank = (int *)d; a.pidx = pidx; a.ppos = ppos;
+      a.hist = hist + q * 256; a.counter = counters + q;
+      a.state = state[q % 3]; a.clear = q > 0 && !final ? state[(q + 2) % 3] : nullptr;
+      a.wstate = wstate; a.wshift = wshift;
+      a.total = total; a.n = n; a.status = S.d_status; a.spin_limit = S.spin_limit;
+    };
+    if (q < key_passes) {
       PassArgs<K, unsigned> a{};
-      a.kin = (const K *)kA; a.vin = iA; a.ain = aA;
-      a.kout = (K *)kB; a.vout = iB; a.aout = aB;
-      a.src = s; a.up = up;
-      a.rank = (int *)d; a.segoff = nullptr; a.pidx = pidx; a.ppos = ppos;
-      a.wstarts = wst; a.wstate = wstate; a.wshift = wshift;
-      a.starts = hist + q * 256; a.state = state; a.counter = counters + q;
-      a.n = n; a.shift = 8 * q; a.status = S.d_status; a.spin_limit = S.spin_limit;
-      if (seg) {
-        launch_pass<K, unsigned, true, IN_ARRAYS, OUT_ARRAYS>(a, tiles);
-      } else if (q == 0) {
-        launch_pass<K, unsigned, false, IN_SRC, OUT_ARRAYS>(a, tiles);
-      } else if (!final) {
-        launch_pass<K, unsigned, false, IN_ARRAYS, OUT_ARRAYS>(a, tiles);
-      } else if (direct) {
-        launch_pass<K, unsigned, false, IN_ARRAYS, OUT_RANK>(a, tiles);
-      } else {
-        launch_pass<K, unsigned, false, IN_ARRAYS, OUT_WIN>(a, tiles);
-      }
+      common(a);
+      a.kin = (const K *)kA; a.kout = (K *)kB; a.ain = aA; a.aout = aB;
+      a.src = s; a.up = up; a.shift = 8 * q;
+      if (seg) launch_pass<K, unsigned, true, IN_ARRAYS, OUT_ARRAYS, true>(a);
+      else if (q == 0) launch_pass<K, unsigned, false, IN_SRC, OUT_ARRAYS, false>(a);
+      else if (!final) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_ARRAYS, false>(a);
+      else if (direct) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_RANK, false>(a);
+      else launch_pass<K, unsigned, false, IN_ARRAYS, OUT_WIN, false>(a);
     } else {
       // segment passes: the segment number is the key, indices ride along
       PassArgs<unsigned, unsigned> a{};
-      const bool first_seg = (q == key_passes);
-      a.kin = first_seg ? aA : (const unsigned *)kA; a.vin = iA; a.ain = nullptr;
-      a.kout = (unsigned *)kB; a.vout = iB; a.aout = nullptr;
-      a.rank = (int *)d; a.segoff = segoff; a.pidx = pidx; a.ppos = ppos;
-      a.wstarts = wst; a.wstate = wstate; a.wshift = wshift;
-      a.starts = hist + q * 256; a.state = state; a.counter = counters + q;
-      a.n = n; a.shift = 8 * (q - key_passes); a.status = S.d_status; a.spin_limit = S.spin_limit;
-      if (!final) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS>(a, tiles);
-      else if (direct) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK>(a, tiles);
-      else launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_WIN>(a, tiles);
+      common(a);
+      a.kin = q == key_passes ? aA : (const unsigned *)kA;
+      a.kout = (unsigned *)kB;
+      a.segbase = segbase; a.shift = 8 * (q - key_passes);
+      if (!final) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS, true>(a);
+      else if (direct) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, true>(a);
+      else launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_WIN, true>(a);
     }
     if (!final) {
-      std::swap(kA, kB); std::swap(iA, iB);
-      if (keypass) std::swap(aA, aB);
+      std::swap(kA, kB);
+      std::swap(iA, iB);
+      if (q < key_passes) std::swap(aA, aB);
     }
   }
   if (!direct) {
-    // (index, position) pairs grouped by window of the index ->
-    // rank[index] = position, one window at a time
-    k_window_scatter<unsigned><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>((unsigned *)d, pidx, (const unsigned *)ppos, n,
-                                                               nullptr);
-    launch_check("k_window_scatter");
+    if (seg)
+      k_rank_scatter<true><<<sc_grid(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, total, wstate,
+                                                                  rk_tile(n));
+    else
+      k_rank_scatter<false><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, nullptr, nullptr,
+                                                                     rk_tile(n));
+    launch_check("k_rank_scatter");
   }
 }
 

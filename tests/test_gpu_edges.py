@@ -21,3 +21,71 @@ def test_rand_group_edges(gpu, oracle, n):
     r = W.rng(n % 9973)
     bounds = r.integers(1, 2 ** 31, size=n, dtype=np.int64).astype(np.int32)
     assert np.array_equal(ops.rand_u(gpu, bounds, seed=n + 5), ops.rand_u(oracle, bounds, seed=n + 5))
+
+
+# ----------------------------------------------------------------- ranks ---
+# sizes of neslgpu_gb300/csrc/rank.cuh and rank.cu: a CTA's segments start in
+# 2048 elements and hold at most 2048; one CTA ranks a whole vector of 4096;
+# digit passes take small tiles up to 2^20 and write ranks by window past 2^23
+LR_T = LR_MAX = 2048
+
+
+def _keys(r, n, typ, dist):
+    if dist == "few":
+        x = r.integers(0, 5, size=n)
+    elif dist == "equal":
+        x = np.full(n, -7)
+    elif dist == "clusters":  # two narrow ranges far apart: crowded buckets
+        x = np.where(r.random(n) < 0.5, r.integers(-40, 40, size=n), 2 ** 31 - 1 - r.integers(0, 900, size=n))
+    else:
+        x = W.int32_uniform(r, n) if typ == "z" else W.float64_normal(r, n)
+    x = np.asarray(x, dtype=np.float64 if typ == "d" else np.int32)
+    if typ == "d" and dist == "special":
+        x[r.random(n) < 0.2] = np.inf
+        x[r.random(n) < 0.2] = -np.inf
+        x[r.random(n) < 0.1] = 0.0
+        x[r.random(n) < 0.1] = -0.0
+        x[r.random(n) < 0.1] *= 2.0 ** -1030
+    return x
+
+
+def _segments(r, shape):
+    if shape == "ones":
+        return np.ones(LR_T * 2 + 5, dtype=np.int32)
+    if shape == "limit":  # around the longest segment one CTA takes, at every place in a tile
+        return np.array([2047, 1, 2048, 3, 2049, 0, 2048, 2048, 1, 4097, 2049, 0, 5, 2046], dtype=np.int32)
+    if shape == "long":  # long segments over several tiles among short ones
+        s = W.geometric_lengths(r, 60_000, 20)
+        return np.insert(s, [3, 3, 900, len(s)], [30_001, 2049, 70_000, 9_000]).astype(np.int32)
+    if shape == "empties":
+        return W.with_empty(r, W.geometric_lengths(r, 50_001, 300), 0.3)
+    if shape == "whole":
+        return W.with_empty(r, W.geometric_lengths(r, 4096, 64), 0.2)
+    return W.lognormal_lengths(r, 400_003, 5, 2, 1 << 18)
+
+
+@pytest.mark.parametrize("shape", ["ones", "limit", "long", "empties", "whole", "lognormal"])
+@pytest.mark.parametrize("dist", ["uniform", "few", "equal", "clusters", "special"])
+@pytest.mark.parametrize("name", ["rku_lez", "rkd_lez", "rku_led", "rkd_led"])
+def test_rank_segments(gpu, oracle, name, dist, shape):
+    r = W.rng(sum(map(ord, name + dist + shape)))
+    lens = _segments(r, shape)
+    x = _keys(r, int(lens.sum()), name[-1], dist)
+    assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 2047, 2049, 4095, 4096, 4097, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("name,dist", [("rku_luz", "uniform"), ("rkd_luz", "few"), ("rku_lud", "special"),
+                                       ("rkd_lud", "uniform"), ("rku_luz", "clusters")])
+def test_rank_whole_vectors(gpu, oracle, name, dist, n):
+    x = _keys(W.rng(n + len(dist)), n, name[-1], dist)
+    assert np.array_equal(ops.rank_u(gpu, name, x), ops.rank_u(oracle, name, x))
+
+
+@pytest.mark.parametrize("name,n", [("rku_lez", (1 << 23) + 1), ("rkd_led", (1 << 23) + 12_345)])
+def test_rank_long_segments_by_window(gpu, oracle, name, n):
+    """Past 2^23 elements the long segments' ranks go through windows of the index that they fill only in part."""
+    r = W.rng(n)
+    lens = W.bimodal_lengths(r, n)
+    x = _keys(r, n, name[-1], "uniform")
+    assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
