@@ -516,6 +516,99 @@ template <class T> void lw_fix_seg(T *d, const T *s, const LwMem &L, const int *
   lw_fix<T>(d, s, L, L.gd, nullptr, ss.n, sdd.n);
 }
 
+// ------------------------------------------------- put by owner ---
+// The same scatters while the destinations' owners fit L2: pass 1 finds every
+// destination's last source position (atomicMax; no value moves and nothing
+// has to be known about repeats), pass 2 walks the destinations in order and
+// takes each owner's value or the default.  Three launches whatever the
+// indices are, the destination is written once and in order, and the default
+// is not copied first.  Pass 1 is bound by one L2 atomic per element (5 M
+// random destinations of 15 M: 41 us), pass 2 by its traffic and the random
+// reads of s.  The check-scatter-fix form above took 10 to 12 launches, a
+// copy of the default, a random atomic per element for the check and, when a
+// destination did repeat, two more random passes.  dpe_pu*, int / float64, us:
+//   n      n_d     ascending            unique               repeated
+//   2^10   3 n      30 /  29 -> 12/ 12   30/  30 ->  12/ 12    30/  31 ->  12/ 12
+//   2^20   3 n      55 /  58 -> 19/ 22   74/  76 ->  24/ 26   113/ 115 ->  25/ 27
+//   2^22   3 n     109 / 147 -> 44/ 61  187/ 257 ->  67/ 84   300/ 416 ->  66/ 82
+//   2^24   3 n     261 / 390 ->212/271  574/ 791 -> 576/743  1759/2039 -> 563/713
+// The line lies at the last row: beyond it the owners are far larger than L2,
+// and each of unique destinations' atomics is a DRAM read-modify-write of a
+// sector where the form above only sets a bit.
+constexpr long PUT_OWNER_MAX = 3L << 24;
+inline bool put_by_owner(long n_d) { return n_d <= PUT_OWNER_MAX; }
+inline size_t put_bytes(long n_d) { return align_up((size_t)n_d * 4, 256) + 256; }
+__global__ void __launch_bounds__(VBLOCK) k_put_owner(const int *__restrict__ idx, const int *__restrict__ f, long n,
+                                                      long n_d, int *__restrict__ owner) {
+  const long i0 = (long)blockIdx.x * (VBLOCK * GITEMS) + threadIdx.x;
+  int g[GITEMS];
+  bool ok[GITEMS];
+#pragma unroll
+  for (int u = 0; u < GITEMS; u++) {
+    const long k = i0 + (long)u * VBLOCK;
+    ok[u] = k < n;
+    g[u] = ok[u] ? __ldcs(idx + k) : -1;
+    if (f && ok[u]) ok[u] = __ldcs(f + k) != 0;
+  }
+#pragma unroll
+  for (int u = 0; u < GITEMS; u++)
+    if (ok[u] && g[u] >= 0 && g[u] < n_d) atomicMax(owner + g[u], (int)(i0 + (long)u * VBLOCK));
+}
+// the segmented forms: the destination of k is off_d[segment of k] + i[k]
+struct PutOwnerSeg {
+  const int *i; const int *f; const int *off_d; int m_d; long n_d; int *owner;
+  __device__ void operator()(int k, int sg, int) const {
+    if (sg < m_d && (f == nullptr || __ldg(f + k))) {
+      const long g = (long)__ldg(off_d + sg) + __ldg(i + k);
+      if (g >= 0 && g < n_d) atomicMax(owner + g, k);
+    }
+  }
+};
+// d[j] = s[owner[j]], or v[j] where nobody writes (v null or d itself: d[j] stays)
+template <class T>
+__global__ void __launch_bounds__(VBLOCK) k_put_take(T *d, const T *__restrict__ s, const T *v,
+                                                     const int *__restrict__ owner, long n_d) {
+  const long j0 = (long)blockIdx.x * (VBLOCK * GITEMS) + threadIdx.x;
+  int w[GITEMS];
+  T x[GITEMS];
+#pragma unroll
+  for (int u = 0; u < GITEMS; u++) {
+    const long j = j0 + (long)u * VBLOCK;
+    w[u] = j < n_d ? __ldcs(owner + j) : -1;
+    if (v && j < n_d) x[u] = __ldcs(v + j);
+  }
+#pragma unroll
+  for (int u = 0; u < GITEMS; u++)
+    if (w[u] >= 0) x[u] = __ldg(s + w[u]);
+#pragma unroll
+  for (int u = 0; u < GITEMS; u++) {
+    const long j = j0 + (long)u * VBLOCK;
+    if (j < n_d && (v || w[u] >= 0)) __stcs(d + j, x[u]);
+  }
+}
+// scratch units of either form
+inline int put_units(long n_s, long n_d, bool seg) {
+  return (int)(((put_by_owner(n_d) ? put_bytes(n_d) : lw_bytes(n_s, n_d, seg)) + 7) / 8);
+}
+// unsegmented when ss is null
+template <class T>
+void put(T *d, const T *s, const int *i, const int *f, const T *v, int n_s, int n_d, const SegView *ss,
+         const SegView *sdd, vec_p scratch, const char *name) {
+  if (n_d <= 0) return;
+  void *mem = scratch_or_work(scratch, put_bytes(n_d));
+  if (!mem) return;
+  int *owner = (int *)align_up((size_t)mem, 256);
+  if (!GCVL_CK(cudaMemsetAsync(owner, 0xFF, (size_t)n_d * 4, stream()))) return;
+  if (ss) {
+    segwalk(PutOwnerSeg{i, f, sdd->off, sdd->m, n_d, owner}, *ss, name);
+  } else {
+    k_put_owner<<<grid_for(n_s, VBLOCK * GITEMS), VBLOCK, 0, stream()>>>(i, f, n_s, n_d, owner);
+    launch_check(name);
+  }
+  k_put_take<T><<<grid_for(n_d, VBLOCK * GITEMS), VBLOCK, 0, stream()>>>(d, s, v == d ? nullptr : v, owner, n_d);
+  launch_check(name);
+}
+
 template <class T> struct BFPerm {  // d[k] = f[k] ? s[i[k]] : 0
   T *d; const T *s; const int *i; const int *f;
   __device__ void operator()(long k) const { d[k] = __ldg(f + k) ? __ldg(s + __ldg(i + k)) : (T)0; }
@@ -900,6 +993,11 @@ META_SEG(ind_lez, INPLACE_NONE)
                              int len_dest, vec_p scratch) {                             \
     ensure_init();                                                                      \
     if (len_src <= 0) return;                                                           \
+    if (put_by_owner(len_dest)) {                                                       \
+      put<T>((T *)d, (const T *)s, (const int *)i, (const int *)f, nullptr, len_src, len_dest, nullptr, nullptr, \
+             scratch, "fpm_pu" #L);                                                     \
+      return;                                                                           \
+    }                                                                                   \
     void *mem = scratch_or_work(scratch, lw_bytes(len_src, len_dest, false));           \
     if (!mem) return;                                                                   \
     const LwMem W = lw_carve(mem, len_src, len_dest, false);                            \
@@ -908,7 +1006,7 @@ META_SEG(ind_lez, INPLACE_NONE)
     lw_fix<T>((T *)d, (const T *)s, W, (const int *)i, (const int *)f, len_src, len_dest); \
   }                                                                                     \
   GCVL_EXPORT int fpm_pu##L##_scratch(int len_src, int len_dest) {                      \
-    return (int)((lw_bytes(len_src, len_dest, false) + 7) / 8);                         \
+    return put_units(len_src, len_dest, false);                                         \
   }                                                                                     \
   GCVL_EXPORT unsigned fpm_pu##L##_inplace(void) { return INPLACE_NONE; }               \
   GCVL_EXPORT void fpm_pe##L(vec_p d, vec_p s, vec_p i, vec_p f, vec_p sd_s, int n_s,   \
@@ -916,16 +1014,21 @@ META_SEG(ind_lez, INPLACE_NONE)
     ensure_init();                                                                      \
     if (m_s == 1) { fpm_pu##L(d, s, i, f, n_s, n_d, scratch); return; }                 \
     if (n_s <= 0) return;                                                               \
+    SegView sdd = seg_view(sd_d, n_d, m_d), ss = seg_view(sd_s, n_s, m_s);              \
+    if (put_by_owner(n_d)) {                                                            \
+      put<T>((T *)d, (const T *)s, (const int *)i, (const int *)f, nullptr, n_s, n_d, &ss, &sdd, scratch, \
+             "fpm_pe" #L);                                                              \
+      return;                                                                           \
+    }                                                                                   \
     void *mem = scratch_or_work(scratch, lw_bytes(n_s, n_d, true));                     \
     if (!mem) return;                                                                   \
     const LwMem W = lw_carve(mem, n_s, n_d, true);                                      \
-    SegView sdd = seg_view(sd_d, n_d, m_d), ss = seg_view(sd_s, n_s, m_s);              \
     lw_detect_seg(W, (const int *)i, (const int *)f, ss, sdd);                          \
     segwalk(FPermSeg<T>{(T *)d, (const T *)s, (const int *)i, (const int *)f, sdd.off, m_d}, ss, "fpm_pe" #L); \
     lw_fix_seg<T>((T *)d, (const T *)s, W, (const int *)i, (const int *)f, ss, sdd);    \
   }                                                                                     \
   GCVL_EXPORT int fpm_pe##L##_scratch(int n_s, int m_s, int n_d, int m_d) {             \
-    (void)m_d; return (int)((lw_bytes(n_s, n_d, m_s != 1) + 7) / 8);                    \
+    (void)m_d; return put_units(n_s, n_d, m_s != 1);                                    \
   }                                                                                     \
   GCVL_EXPORT unsigned fpm_pe##L##_inplace(void) { return INPLACE_NONE; }               \
   GCVL_EXPORT void bfp_pu##L(vec_p d, vec_p s, vec_p i, vec_p f, int len_src,           \
@@ -946,6 +1049,11 @@ META_SEG(ind_lez, INPLACE_NONE)
   GCVL_EXPORT void dpe_pu##L(vec_p d, vec_p s, vec_p i, vec_p v, int len_src,           \
                              int len_dest, vec_p scratch) {                             \
     ensure_init();                                                                      \
+    if (len_src > 0 && put_by_owner(len_dest)) {                                        \
+      put<T>((T *)d, (const T *)s, (const int *)i, nullptr, (const T *)v, len_src, len_dest, nullptr, nullptr, \
+             scratch, "dpe_pu" #L);                                                     \
+      return;                                                                           \
+    }                                                                                   \
     copy_dev<T>(d, v, len_dest);                                                        \
     if (len_src <= 0) return;                                                           \
     const size_t lb = lw_bytes(len_src, len_dest, false);                               \
@@ -957,31 +1065,41 @@ META_SEG(ind_lez, INPLACE_NONE)
     lw_fix<T>((T *)d, (const T *)s, W, (const int *)i, nullptr, len_src, len_dest);     \
   }                                                                                     \
   GCVL_EXPORT int dpe_pu##L##_scratch(int len_src, int len_dest) {                      \
-    return (int)((lw_bytes(len_src, len_dest, false) + 7) / 8) + scatter_units<T>(len_src, len_dest); \
+    return put_units(len_src, len_dest, false) + (put_by_owner(len_dest) ? 0 : scatter_units<T>(len_src, len_dest)); \
   }                                                                                     \
   GCVL_EXPORT unsigned dpe_pu##L##_inplace(void) { return INPLACE_3; }                  \
   GCVL_EXPORT void dpe_pe##L(vec_p d, vec_p s, vec_p i, vec_p v, vec_p sd_s, int n_s,   \
                              int m_s, vec_p sd_d, int n_d, int m_d, vec_p scratch) {    \
     ensure_init();                                                                      \
     if (m_s == 1) { dpe_pu##L(d, s, i, v, n_s, n_d, scratch); return; }                 \
+    SegView sdd = seg_view(sd_d, n_d, m_d), ss = seg_view(sd_s, n_s, m_s);              \
+    if (n_s > 0 && put_by_owner(n_d)) {                                                 \
+      put<T>((T *)d, (const T *)s, (const int *)i, nullptr, (const T *)v, n_s, n_d, &ss, &sdd, scratch, \
+             "dpe_pe" #L);                                                              \
+      return;                                                                           \
+    }                                                                                   \
     copy_dev<T>(d, v, n_d);                                                             \
     if (n_s <= 0) return;                                                               \
     void *mem = scratch_or_work(scratch, lw_bytes(n_s, n_d, true));                     \
     if (!mem) return;                                                                   \
     const LwMem W = lw_carve(mem, n_s, n_d, true);                                      \
-    SegView sdd = seg_view(sd_d, n_d, m_d), ss = seg_view(sd_s, n_s, m_s);              \
     lw_detect_seg(W, (const int *)i, nullptr, ss, sdd);                                 \
     segwalk(FPermSeg<T>{(T *)d, (const T *)s, (const int *)i, nullptr, sdd.off, m_d}, ss, "dpe_pe" #L); \
     lw_fix_seg<T>((T *)d, (const T *)s, W, (const int *)i, nullptr, ss, sdd);           \
   }                                                                                     \
   GCVL_EXPORT int dpe_pe##L##_scratch(int n_s, int m_s, int n_d, int m_d) {             \
     (void)m_d;                                                                          \
-    return m_s == 1 ? dpe_pu##L##_scratch(n_s, n_d) : (int)((lw_bytes(n_s, n_d, true) + 7) / 8); \
+    return m_s == 1 ? dpe_pu##L##_scratch(n_s, n_d) : put_units(n_s, n_d, true); \
   }                                                                                     \
   GCVL_EXPORT unsigned dpe_pe##L##_inplace(void) { return INPLACE_3; }                  \
   GCVL_EXPORT void dfp_pu##L(vec_p d, vec_p s, vec_p i, vec_p f, vec_p v, int len_src,  \
                              int len_dest, vec_p scratch) {                             \
     ensure_init();                                                                      \
+    if (len_src > 0 && put_by_owner(len_dest)) {                                        \
+      put<T>((T *)d, (const T *)s, (const int *)i, (const int *)f, (const T *)v, len_src, len_dest, nullptr, \
+             nullptr, scratch, "dfp_pu" #L);                                            \
+      return;                                                                           \
+    }                                                                                   \
     copy_dev<T>(d, v, len_dest);                                                        \
     fpm_pu##L(d, s, i, f, len_src, len_dest, scratch);                                  \
   }                                                                                     \
@@ -991,9 +1109,15 @@ META_SEG(ind_lez, INPLACE_NONE)
                              int n_s, int m_s, vec_p sd_d, int n_d, int m_d,            \
                              vec_p scratch) {                                           \
     ensure_init();                                                                      \
+    if (m_s == 1) { dfp_pu##L(d, s, i, f, v, n_s, n_d, scratch); return; }              \
+    if (n_s > 0 && put_by_owner(n_d)) {                                                 \
+      SegView sdd = seg_view(sd_d, n_d, m_d), ss = seg_view(sd_s, n_s, m_s);            \
+      put<T>((T *)d, (const T *)s, (const int *)i, (const int *)f, (const T *)v, n_s, n_d, &ss, &sdd, scratch, \
+             "dfp_pe" #L);                                                              \
+      return;                                                                           \
+    }                                                                                   \
     copy_dev<T>(d, v, n_d);                                                             \
-    if (m_s == 1) fpm_pu##L(d, s, i, f, n_s, n_d, scratch);                             \
-    else fpm_pe##L(d, s, i, f, sd_s, n_s, m_s, sd_d, n_d, m_d, scratch);                \
+    fpm_pe##L(d, s, i, f, sd_s, n_s, m_s, sd_d, n_d, m_d, scratch);                \
   }                                                                                     \
   GCVL_EXPORT int dfp_pe##L##_scratch(int n_s, int m_s, int n_d, int m_d) {             \
     return fpm_pe##L##_scratch(n_s, m_s, n_d, m_d);                                     \

@@ -89,3 +89,70 @@ def test_rank_long_segments_by_window(gpu, oracle, name, n):
     lens = W.bimodal_lengths(r, n)
     x = _keys(r, n, name[-1], "uniform")
     assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
+
+
+# ------------------------------------------------------------------ puts ---
+# the owner passes take 2048 elements a CTA, up to 3 * 2^24 destinations
+def _put_case(r, n_s, n_d, order):
+    if order == "ascending":
+        return np.sort(r.permutation(n_d)[:n_s]).astype(np.int32)
+    if order == "one":
+        return np.full(n_s, n_d - 1, dtype=np.int32)
+    return r.integers(0, n_d, size=n_s).astype(np.int32)
+
+
+@pytest.mark.parametrize("n_s,n_d", [(1, 1), (5, 3), (2047, 2049), (2048, 2048), (2049, 6000), (3, 100_001)])
+@pytest.mark.parametrize("order", ["ascending", "one", "random"])
+@pytest.mark.parametrize("t", "zbd")
+def test_put_by_owner(gpu, oracle, t, order, n_s, n_d):
+    r = W.rng(n_s * 7 + n_d + ord(t))
+    if order == "ascending" and n_s > n_d:
+        pytest.skip("more values than places")
+    idx = _put_case(r, n_s, n_d, order)
+    x = _keys(r, n_s, t, "few" if t == "b" else "uniform")
+    v = _keys(r, n_d, t, "few" if t == "b" else "uniform")
+    flags = (r.random(n_s) < 0.6).astype(np.int32)
+    for R in (gpu, oracle):
+        R.got = [ops.dpe_u(R, f"dpe_pu{t}", x, idx, v), ops.fpm_u(R, f"fpm_pu{t}", x, idx, flags, n_d, v),
+                 ops.fpm_u(R, f"dfp_pu{t}", x, idx, flags, n_d, v)]
+    for a, b in zip(gpu.got, oracle.got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("t", "zd")
+def test_put_default_in_place(gpu, oracle, t):
+    """The destination may be the default itself."""
+    r = W.rng(77)
+    n_s, n_d = 3001, 9999
+    idx, x, v = _put_case(r, n_s, n_d, "random"), _keys(r, n_s, t, "uniform"), _keys(r, n_d, t, "uniform")
+    c = gpu.cvl
+    d, s, i = gpu.vec(v, t), gpu.vec(x, t), gpu.vec(idx, "z")
+    scr = gpu.units(gpu.fn(f"dpe_pu{t}_scratch")(n_s, n_d))
+    gpu.fn(f"dpe_pu{t}")(d.ptr, s.ptr, i.ptr, d.ptr, n_s, n_d, scr.ptr)
+    assert np.array_equal(gpu.get(d, n_d), ops.dpe_u(oracle, f"dpe_pu{t}", x, idx, v))
+    assert c.gcvl_sync() == 0
+
+
+@pytest.mark.parametrize("t", "zd")
+def test_put_segments(gpu, oracle, t):
+    r = W.rng(78)
+    len_s = W.with_empty(r, W.geometric_lengths(r, 20_011, 9), 0.2)
+    len_d = (len_s * 2 + r.integers(0, 3, size=len_s.size)).astype(np.int32)
+    len_d[len_s > 0] += 1
+    idx = W.seg_indices(r, len_d, len_s)
+    x, v = _keys(r, int(len_s.sum()), t, "uniform"), _keys(r, int(len_d.sum()), t, "uniform")
+    flags = (r.random(x.size) < 0.6).astype(np.int32)
+    for R in (gpu, oracle):
+        R.got = [ops.dpe_e(R, f"dpe_pe{t}", x, idx, v, len_s, len_d),
+                 ops.fpm_e(R, f"fpm_pe{t}", x, idx, flags, len_s, len_d, v),
+                 ops.fpm_e(R, f"dfp_pe{t}", x, idx, flags, len_s, len_d, v)]
+    for a, b in zip(gpu.got, oracle.got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n_d", [3 << 24, (3 << 24) + 1])
+def test_put_either_side_of_the_owner_limit(gpu, oracle, n_d):
+    r = W.rng(n_d)
+    idx = r.integers(0, n_d, size=100_003).astype(np.int32)
+    x, v = _keys(r, idx.size, "z", "uniform"), np.arange(n_d, dtype=np.int32)
+    assert np.array_equal(ops.dpe_u(gpu, "dpe_puz", x, idx, v), ops.dpe_u(oracle, "dpe_puz", x, idx, v))
