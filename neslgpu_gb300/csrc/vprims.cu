@@ -628,108 +628,20 @@ template <class T> void copy_dev(vec_p d, vec_p s, int n) {
 }
 
 // ---------------------------------------------------------------- pack ---
-// Stable compaction in one pass: a CTA counts the true flags of its tile,
-// gets the number of true flags in earlier tiles by decoupled look-back,
-// compacts its kept values in shared memory and writes them as one
-// contiguous, coalesced run.
+// Stable compaction in two passes, no tile waiting for another.  Pass 1 reads
+// the flags once, writes them as a bit mask (element k: bit k&31 of word
+// k>>5) and every tile's count of true flags; pass 2 reads the mask (one bit
+// per element instead of the 4-byte flag) and the values, compacts each tile
+// in shared memory and writes it as one coalesced run at the tile's output
+// offset.  That offset is the sum of the earlier tiles' counts: with at most
+// PACK_SUM_TILES tiles every CTA adds them itself (4 KB from L2 at most),
+// beyond them the library's +-scan of the counts gives it.  A vector of one
+// tile takes pass 2 alone, on its flags.
+// 2^20 int elements: the scan and the cleared area it needs took 6 us of 15.
 constexpr int PBLOCK = 256, PITEMS = 16, PTILE = PBLOCK * PITEMS;
-
-template <class T>
-__global__ void __launch_bounds__(PBLOCK) k_pack(T *__restrict__ d, const T *__restrict__ s,
-                                                const int *__restrict__ f, int n, LookbackMem lb,
-                                                unsigned *status, int spin_limit) {
-  constexpr int PE = 32;  // padding period of the int staging buffer
-  __shared__ int s_rank[PTILE + PTILE / PE];
-  __shared__ T s_val[PTILE];
-  __shared__ int s_wsum[PBLOCK / 32];
-  __shared__ int s_prefix, s_count;
-  __shared__ unsigned s_tile;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(lb.counter, 1u);
-  __syncthreads();
-  const int tile = (int)s_tile;
-  const long base = (long)tile * PTILE;
-  const int valid = (int)min((long)PTILE, (long)n - base);
-
-  // values: coalesced striped loads issued first, kept in registers until
-  // their ranks are known (so their latency overlaps the ranking)
-  T vals[PITEMS];
-#pragma unroll
-  for (int j = 0; j < PITEMS; j++) {
-    int e = j * PBLOCK + tid;
-    if (e < valid) vals[j] = __ldcs(s + base + e);
-  }
-  // flags: coalesced striped loads, transposed to 16 consecutive per thread
-  const int wbase = warp * 32 * PITEMS;
-#pragma unroll
-  for (int j = 0; j < PITEMS; j++) {
-    int e = wbase + j * 32 + lane;
-    s_rank[e + e / PE] = (e < valid) ? (__ldcs(f + base + e) != 0) : 0;
-  }
-  __syncwarp();
-  unsigned bits = 0;
-#pragma unroll
-  for (int i = 0; i < PITEMS; i++) {
-    int e = tid * PITEMS + i;
-    bits |= (unsigned)s_rank[e + e / PE] << i;
-  }
-  // exclusive scan of the per-thread counts across the CTA
-  int c = __popc(bits), incl = c;
-#pragma unroll
-  for (int dd = 1; dd < 32; dd <<= 1) {
-    int o = shfl_up(incl, dd);
-    if (lane >= dd) incl += o;
-  }
-  if (lane == 31) s_wsum[warp] = incl;
-  __syncthreads();
-  int wpre = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < PBLOCK / 32; w++) {
-    int v = s_wsum[w];
-    if (w < warp) wpre += v;
-    total += v;
-  }
-  int r = wpre + incl - c;
-  // rank of every element within the tile's output (-1 when dropped)
-#pragma unroll
-  for (int i = 0; i < PITEMS; i++) {
-    int e = tid * PITEMS + i;
-    s_rank[e + e / PE] = ((bits >> i) & 1u) ? r++ : -1;
-  }
-
-  // decoupled look-back over tile counts (int add, no segments)
-  if (warp == 0) {
-    if (lane == 0) lb_publish(lb.word + tile, tile == 0 ? TS_INC : TS_AGG, (unsigned long long)(unsigned)total);
-    int P = 0;
-    if (tile > 0) {
-      P = lookback_prefix<AddZ>(lb.word, tile, status, spin_limit);
-      if (lane == 0) lb_publish(lb.word + tile, TS_INC, (unsigned long long)(unsigned)(P + total));
-    }
-    if (lane == 0) { s_prefix = (int)P; s_count = total; }
-  }
-  __syncthreads();
-  // values: coalesced striped loads, placed at their rank in shared memory
-#pragma unroll
-  for (int j = 0; j < PITEMS; j++) {
-    int e = j * PBLOCK + tid;
-    int rk = e < valid ? s_rank[e + e / PE] : -1;
-    if (rk >= 0) s_val[rk] = vals[j];
-  }
-  __syncthreads();
-  const long out0 = s_prefix;
-  const int cnt = s_count;
-  for (int e = tid; e < cnt; e += PBLOCK) d[out0 + e] = s_val[e];
-}
-
-// Pack of long vectors in two passes, no tile waiting for another (at large
-// n the one-pass kernel's look-back chain, not HBM, bounds it).  Pass 1
-// reads the flags once, writes them as a bit mask (element k: bit k&31 of
-// word k>>5) and every tile's count of true flags; an exclusive +-scan of
-// the counts gives each tile its output offset; pass 2 reads the mask (one
-// bit per element instead of the 4-byte flag) and the values, and writes
-// each tile's kept values as one coalesced run.
-constexpr int PACK_TWO_PASS_TILES = 64;
+constexpr int PACK_SUM_TILES = 1024;
 constexpr int PWORDS = PTILE / 32;  // mask words per tile
+enum { PACK_ALONE = 0, PACK_SUM = 1, PACK_SCANNED = 2 };
 
 __global__ void __launch_bounds__(PBLOCK) k_pack_count(const int *__restrict__ f, int n,
                                                       unsigned *__restrict__ bits, int *__restrict__ cnt) {
@@ -764,14 +676,16 @@ __global__ void __launch_bounds__(PBLOCK) k_pack_count(const int *__restrict__ f
   }
 }
 
-template <class T>
+// at: PACK_SUM the tiles' counts, PACK_SCANNED their offsets
+template <class T, int FORM>
 __global__ void __launch_bounds__(PBLOCK) k_pack_place(T *__restrict__ d, const T *__restrict__ s,
-                                                      const unsigned *__restrict__ bits,
-                                                      const int *__restrict__ offs, int n) {
+                                                      const int *__restrict__ f, const unsigned *__restrict__ bits,
+                                                      const int *__restrict__ at, int n) {
   __shared__ T s_val[PTILE];
   __shared__ unsigned s_word[PWORDS];
   __shared__ int s_wpre[PWORDS + 1];
   __shared__ int s_ws[PWORDS / 32];
+  __shared__ int s_sum[PBLOCK / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long base = (long)blockIdx.x * PTILE;
   const int valid = (int)min((long)PTILE, (long)n - base);
@@ -782,11 +696,26 @@ __global__ void __launch_bounds__(PBLOCK) k_pack_place(T *__restrict__ d, const 
     const int e = j * PBLOCK + tid;
     if (e < valid) vals[j] = __ldcs(s + base + e);
   }
-  const long out0 = __ldg(offs + blockIdx.x);
+  long out0 = FORM == PACK_SCANNED ? __ldg(at + blockIdx.x) : 0;
+  if constexpr (FORM == PACK_SUM) {
+    int sum = 0;
+    for (int t = tid; t < (int)blockIdx.x; t += PBLOCK) sum += __ldg(at + t);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_sum[warp] = sum;
+  }
+  if constexpr (FORM == PACK_ALONE) {  // the mask from the flags
+#pragma unroll
+    for (int j = 0; j < PITEMS; j++) {
+      const int e = j * PBLOCK + tid;
+      const unsigned b = __ballot_sync(0xffffffffu, e < valid && __ldcs(f + e) != 0);
+      if (lane == 0) s_word[e >> 5] = b;
+    }
+    __syncthreads();
+  }
   // exclusive prefix of the words' popcounts (threads 0..PWORDS-1, one word each)
   if (tid < PWORDS) {
     const int nw = (valid + 31) >> 5;
-    const unsigned w = tid < nw ? __ldg(bits + (base >> 5) + tid) : 0u;
+    const unsigned w = FORM == PACK_ALONE ? s_word[tid] : tid < nw ? __ldg(bits + (base >> 5) + tid) : 0u;
     const int c = __popc(w);
     int incl = c;
 #pragma unroll
@@ -807,6 +736,10 @@ __global__ void __launch_bounds__(PBLOCK) k_pack_place(T *__restrict__ d, const 
     if (tid == PWORDS - 1) s_wpre[PWORDS] = p + s_ws[warp];
   }
   __syncthreads();
+  if constexpr (FORM == PACK_SUM) {
+#pragma unroll
+    for (int w = 0; w < PBLOCK / 32; w++) out0 += s_sum[w];
+  }
   const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
   for (int j = 0; j < PITEMS; j++) {
@@ -838,34 +771,28 @@ template <class T> void pack(vec_p d, vec_p s, vec_p f, int n, vec_p scratch, co
   ensure_init();
   State &S = st();
   if (n <= 0) return;
-  int tiles = ceil_div(n, PTILE);
-  if (tiles >= PACK_TWO_PASS_TILES) {
-    const PackLayout L = pack_layout(n);
-    char *mem = (char *)scratch_or_work(scratch, L.total);
-    if (!mem) return;
-    unsigned *bits = (unsigned *)(mem + L.bits);
-    int *cnt = (int *)(mem + L.cnt), *offs = (int *)(mem + L.offs);
-    k_pack_count<<<tiles, PBLOCK, 0, S.stream>>>((const int *)f, n, bits, cnt);
-    launch_check(name);
-    add_suz(offs, cnt, tiles, mem + L.scan);
-    k_pack_place<T><<<tiles, PBLOCK, 0, S.stream>>>((T *)d, (const T *)s, bits, offs, n);
+  const int tiles = ceil_div(n, PTILE);
+  if (tiles == 1) {
+    k_pack_place<T, PACK_ALONE><<<1, PBLOCK, 0, S.stream>>>((T *)d, (const T *)s, (const int *)f, nullptr, nullptr, n);
     launch_check(name);
     return;
   }
-  void *mem = scratch_or_work(scratch, lookback_bytes(tiles));
+  const PackLayout L = pack_layout(n);
+  char *mem = (char *)scratch_or_work(scratch, L.total);
   if (!mem) return;
-  LookbackMem lb = lookback_carve(mem, tiles);
-  GCVL_CK(cudaMemsetAsync(mem, 0, lookback_clear_bytes(tiles), S.stream));
-  k_pack<T><<<tiles, PBLOCK, 0, S.stream>>>((T *)d, (const T *)s, (const int *)f, n, lb, S.d_status,
-                                            S.spin_limit);
+  unsigned *bits = (unsigned *)(mem + L.bits);
+  int *cnt = (int *)(mem + L.cnt), *offs = (int *)(mem + L.offs);
+  k_pack_count<<<tiles, PBLOCK, 0, S.stream>>>((const int *)f, n, bits, cnt);
+  launch_check(name);
+  if (tiles <= PACK_SUM_TILES) {
+    k_pack_place<T, PACK_SUM><<<tiles, PBLOCK, 0, S.stream>>>((T *)d, (const T *)s, nullptr, bits, cnt, n);
+  } else {
+    add_suz(offs, cnt, tiles, mem + L.scan);
+    k_pack_place<T, PACK_SCANNED><<<tiles, PBLOCK, 0, S.stream>>>((T *)d, (const T *)s, nullptr, bits, offs, n);
+  }
   launch_check(name);
 }
-int pack_units(int n) {
-  if (n <= 0) return 0;
-  const int tiles = ceil_div(n, PTILE);
-  if (tiles >= PACK_TWO_PASS_TILES) return (int)((pack_layout(n).total + 7) / 8);
-  return lookback_units(tiles);
-}
+int pack_units(int n) { return n <= PTILE ? 0 : (int)((pack_layout(n).total + 7) / 8); }
 
 }  // namespace gcvl
 

@@ -156,3 +156,75 @@ def test_put_either_side_of_the_owner_limit(gpu, oracle, n_d):
     idx = r.integers(0, n_d, size=100_003).astype(np.int32)
     x, v = _keys(r, idx.size, "z", "uniform"), np.arange(n_d, dtype=np.int32)
     assert np.array_equal(ops.dpe_u(gpu, "dpe_puz", x, idx, v), ops.dpe_u(oracle, "dpe_puz", x, idx, v))
+
+
+# ----------------------------------- one-launch forms of scans and friends ---
+# one tile: 4096 ints, 2048 doubles; segment descriptors: ranges of 8192
+# elements, 4096 lengths scanned in the CTA; packs: tiles of 4096, 1024 summed
+def _lens(r, n, shape):
+    if shape == "one-element":
+        return np.ones(n, dtype=np.int32)
+    if shape == "long":
+        return np.array([0, n - n // 3, 0, 0, n // 3, 0], dtype=np.int32)
+    return W.with_empty(r, W.geometric_lengths(r, n, 37), 0.3)
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 2047, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 300_007])
+@pytest.mark.parametrize("shape", ["one-element", "long", "geometric"])
+def test_segmented_at_tile_edges(gpu, oracle, shape, n):
+    r = W.rng(n * 3 + len(shape))
+    lens = _lens(r, n, shape)
+    assert int(lens.sum()) == n
+    xi, xb = W.int32_uniform(r, n), (r.random(n) < 0.4).astype(np.int32)
+    xd = W.float64_normal(r, n)
+    for R in (gpu, oracle):
+        R.got = [ops.scan_e(R, "add_sez", xi, lens), ops.scan_e(R, "max_sed", xd, lens), ops.scan_e(R, "xor_seb", xb, lens),
+                 ops.reduce_e(R, "max_rez", xi, lens), ops.reduce_e(R, "min_red", xd, lens),
+                 ops.reduce_e(R, "ior_reb", xb, lens), ops.pk1_e(R, xb, lens), *ops.pack_e(R, "pk2_lez", xi, xb, lens),
+                 *ops.pack_e(R, "pk2_led", xd, xb, lens), ops.dis_e(R, "dis_vez", np.arange(lens.size), lens)]
+    for k, (a, b) in enumerate(zip(gpu.got, oracle.got)):
+        assert np.array_equal(a, b), k
+    # sums within 1e-12 of the magnitudes summed, as for every float64 sum
+    start = np.cumsum(lens) - lens
+    c = np.concatenate([[0.0], np.cumsum(np.abs(xd))])
+    mag = c[start + lens] - c[start]
+    g, o = ops.reduce_e(gpu, "add_red", xd, lens), ops.reduce_e(oracle, "add_red", xd, lens)
+    assert np.all(np.abs(g - o) <= 1e-12 * mag)
+    g, o = ops.scan_e(gpu, "add_sed", xd, lens), ops.scan_e(oracle, "add_sed", xd, lens)
+    assert np.all(np.abs(g - o) <= 1e-12 * np.repeat(mag, lens))
+
+
+@pytest.mark.parametrize("m,n", [(4096, 5000), (4097, 5000), (4096, 2 ** 22 + 17), (3, 8192 * 304), (3, 8192 * 304 + 1),
+                                 (1, 8192), (5, 0)])
+def test_segment_descriptor_forms(gpu, oracle, m, n):
+    """Either side of the lengths and the elements that the one-launch form takes."""
+    r = W.rng(m + n)
+    cut = np.sort(r.integers(0, n + 1, size=m - 1))
+    lens = np.diff(np.concatenate([[0], cut, [n]])).astype(np.int32)
+    x = W.int32_uniform(r, n)
+    for R in (gpu, oracle):
+        R.got = [ops.scan_e(R, "add_sez", x, lens), ops.reduce_e(R, "max_rez", x, lens),
+                 ops.dis_e(R, "dis_vez", np.arange(m), lens)]
+    for a, b in zip(gpu.got, oracle.got):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 511, 512, 513, 8191, 8192, 8193, 4096 * 1024, 4096 * 1024 + 1])
+def test_reduce_and_pack_edges(gpu, oracle, n):
+    r = W.rng(n)
+    x, f = W.int32_uniform(r, n), (r.random(n) < 0.5).astype(np.int32)
+    for name in ("add_ruz", "min_ruz", "xor_ruz"):
+        assert ops.reduce_u(gpu, name, x) == ops.reduce_u(oracle, name, x)
+    assert ops.pk1_u(gpu, f) == ops.pk1_u(oracle, f)
+    assert np.array_equal(ops.pack_u(gpu, "pk2_luz", x, f), ops.pack_u(oracle, "pk2_luz", x, f))
+
+
+@pytest.mark.parametrize("ranges", [1, 2, 1024, 1025, 2049])
+def test_reduction_fix_up_by_one_cta_or_several(gpu, oracle, ranges):
+    """One segment over every tile but the ends: each tile's result needs the tiles before it."""
+    n = ranges * 2048 + 3
+    lens = np.array([2, n - 3, 1], dtype=np.int32)
+    x = W.rng(ranges).integers(-9, 10, size=n).astype(np.float64)  # sums exact in any order
+    for name in ("add_red", "max_red"):
+        assert np.array_equal(ops.reduce_e(gpu, name, x, lens), ops.reduce_e(oracle, name, x, lens))
+    assert np.array_equal(ops.reduce_e(gpu, "add_rez", x, lens), ops.reduce_e(oracle, "add_rez", x, lens))
