@@ -166,11 +166,14 @@ def _lens(r, n, shape):
         return np.ones(n, dtype=np.int32)
     if shape == "long":
         return np.array([0, n - n // 3, 0, 0, n // 3, 0], dtype=np.int32)
+    if shape in ("fours", "fives"):  # either side of the mean from which warps reduce ranges of their own
+        k = 4 if shape == "fours" else 5
+        return np.array([k] * (n // k) + [n % k] * (n % k > 0), dtype=np.int32)
     return W.with_empty(r, W.geometric_lengths(r, n, 37), 0.3)
 
 
-@pytest.mark.parametrize("n", [1, 63, 64, 65, 2047, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 300_007])
-@pytest.mark.parametrize("shape", ["one-element", "long", "geometric"])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 2047, 2048, 2049, 2559, 2561, 4095, 4096, 4097, 8191, 8192, 8193, 300_007])
+@pytest.mark.parametrize("shape", ["one-element", "fours", "fives", "long", "geometric"])
 def test_segmented_at_tile_edges(gpu, oracle, shape, n):
     r = W.rng(n * 3 + len(shape))
     lens = _lens(r, n, shape)
