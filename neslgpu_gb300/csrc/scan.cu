@@ -433,15 +433,30 @@ template <int MODE> constexpr int cta_threads() { return MODE == M_REDUCE ? TT :
 template <int MODE, class T, bool GATHER> constexpr int tma_minb() {
   return GATHER ? 4 : MODE == M_REDUCE ? (sizeof(T) == 8 ? GCVL_RED_MINB_D : GCVL_RED_MINB_Z) : GCVL_SCAN_MINB;
 }
-template <class Op, int MODE, bool SEG, bool CHAIN = false, bool GATHER = false>
+// STAGE (reductions of segments of hardly more than one element): the tile's
+// results -- one per segment that ends in the tile, consecutive ones -- are
+// put together in shared memory, where the tile was, and leave as one
+// coalesced run.  Stored by the threads that find them, one-element segments
+// make every lane of a store hit a line of its own.  At 2^25 elements, stored
+// directly / staged, us: mean 1 max_rez 271 / 144, add_red 257 / 195, mul_red
+// 271 / 170; mean 1.3 164 / 140, 205 / 196, 181 / 176 (max_red 210 / 215);
+// mean 2 115 / 127, 173 / 183, 148 / 157; mean 4 86 / 106, 167 / 178, 141 /
+// 149.  Hence the lines at means 1.5 (4-byte) and 1.25 (8-byte); and from two
+// tiles per SM on, because fewer tiles only pay for the extra barrier (2^18
+// elements 14.4 / 15.5).
+template <class T> inline bool red_staged(long n, long m, long tiles) {
+  return tiles > 2L * st().sm_count && (sizeof(T) == 4 ? 2 * n < 3 * m : 4 * n < 5 * m);
+}
+template <class Op, int MODE, bool SEG, bool CHAIN = false, bool GATHER = false, bool STAGE = false>
 __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename Op::T, GATHER>()) k_scan_tma(const __grid_constant__ CUtensorMap tin,
                                                      const __grid_constant__ CUtensorMap tout,
                                                      TArgs<typename Op::T> a) {
   typedef typename Op::T T;
   constexpr int ITEMS = row_items<T>(), TILE = TT * ITEMS, NW = TT / 32;
+  constexpr int STAGE_PAD = STAGE ? TILE / 32 : 0;  // a staged run holds a word per 32 results between them, as wpad()
   extern __shared__ unsigned char dyn_smem[];
   unsigned char *tile_b = (unsigned char *)(((size_t)dyn_smem + 1023) & ~(size_t)1023);
-  int *win = (int *)(tile_b + TILE * sizeof(T));
+  int *win = (int *)(tile_b + (TILE + STAGE_PAD) * sizeof(T));
   __shared__ unsigned long long bar;
   __shared__ int s_wf[NW], s_wpf[NW];
   __shared__ T s_wv[NW], s_wpv[NW];
@@ -504,10 +519,17 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
   // reductions also need segment numbers: a window of offsets whose bounds
   // come straight from the granule table (tiles start on granule boundaries)
   int W = 0, sf = 0;
+  int out_s0 = 0, out_cnt = 0;  // STAGE: the segments that end in this tile
+  bool staged = false;
   if (SEG && MODE == M_REDUCE) {
     sf = __ldg(a.sv.gran + base / kGranule);
     const long e = base + valid;
     const int sl = (e >= a.n) ? a.sv.m - 1 : __ldg(a.sv.gran + e / kGranule);
+    if constexpr (STAGE) {
+      out_s0 = tile == 0 ? 0 : sf;
+      out_cnt = (e >= a.n ? a.sv.m : sl) - out_s0;
+      staged = out_cnt <= TILE;
+    }
     W = sl - sf + 2;
     if (W <= a.wmax)
       for (int i = tid; i < W; i += TT) win[wpad(i)] = __ldg(a.sv.off + sf + i);
@@ -580,6 +602,18 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
     }
   }
 
+  // where a result goes: its place in the staged run, or the output itself
+  T *const stage = (T *)tile_b;
+  auto put = [&](int s, T v) {
+    if (STAGE && staged) {
+      const int q = s - out_s0;
+      stage[wpad(q)] = v;
+    } else {
+      a.out[s] = v;
+    }
+  };
+  if constexpr (STAGE) named_sync(2, TT);  // every row is read: the tile's place is free
+
   int tf;
   T tv;
   // Reductions other than float64 + take one pass over the thread's items:
@@ -596,7 +630,7 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
     if (cnt > 0) {
       const int m = a.sv.m;
       if (k0 == 0)
-        for (int q = 0; q < s0; q++) a.out[q] = Op::init();  // empty segments before element 0
+        for (int q = 0; q < s0; q++) put(q, Op::init());  // empty segments before element 0
       int sg = s0;
       int end = off(sg + 1);
 #pragma unroll
@@ -605,10 +639,10 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
           if ((heads >> i) & 1u) { r = Op::init(); started = true; }
           r = Op::apply(r, x[i]);
           if (k0 + i + 1 == end) {
-            if (started) a.out[sg] = r;
+            if (started) put(sg, r);
             else { first_s = sg; first_v = r; }
             int s2 = sg + 1;
-            while (s2 < m && off(s2 + 1) == end) { a.out[s2] = Op::init(); ++s2; }
+            while (s2 < m && off(s2 + 1) == end) { put(s2, Op::init()); ++s2; }
             sg = s2;
             if (sg < m) end = off(sg + 1);
           }
@@ -698,7 +732,7 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
     }
   } else if constexpr (ONE_PASS) {  // the one result still lacking the earlier part
     if (first_s >= 0) {
-      a.out[first_s] = Op::apply(run, first_v);
+      put(first_s, Op::apply(run, first_v));
       if (!pf) a.lead[tile] = first_s;  // began in an earlier tile
     }
   } else {  // M_REDUCE: results at segment ends
@@ -721,7 +755,7 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
     if (cnt > 0) {
       const int m = a.sv.m;
       if (k0 == 0)
-        for (int s = 0; s < s0; s++) a.out[s] = Op::init();
+        for (int s = 0; s < s0; s++) put(s, Op::init());
       int s = s0;
       int end = off(s + 1);
       if constexpr (std::is_same<Op, AddD>::value) {
@@ -735,10 +769,10 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
               if ((heads >> i) & 1u) r = 0.0;
               r = __dadd_rn(r, x[i]);
               if ((ends >> i) & 1u) {
-                a.out[s] = r;
+                put(s, r);
                 if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
                 int s2 = s + 1;
-                while (s2 < m && off(s2 + 1) == end) { a.out[s2] = 0.0; ++s2; }
+                while (s2 < m && off(s2 + 1) == end) { put(s2, 0.0); ++s2; }
                 s = s2;
                 if (s < m) end = off(s + 1);
               }
@@ -752,10 +786,10 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
           ends &= ends - 1;
           {
             double pv2 = fx_range<ITEMS>(x, ps, i + 1);
-            a.out[s] = ((heads >> ps) & 1u) ? pv2 : AddD::apply(run, pv2);
+            put(s, ((heads >> ps) & 1u) ? pv2 : AddD::apply(run, pv2));
             if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
             int s2 = s + 1;
-            while (s2 < m && off(s2 + 1) == end) { a.out[s2] = 0.0; ++s2; }
+            while (s2 < m && off(s2 + 1) == end) { put(s2, 0.0); ++s2; }
             s = s2;
             if (s < m) end = off(s + 1);
             ps = i + 1;
@@ -768,16 +802,22 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
             if ((heads >> i) & 1u) run = Op::init();
             run = Op::apply(run, x[i]);
             if (k0 + i + 1 == end) {
-              a.out[s] = run;
+              put(s, run);
               if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
               int s2 = s + 1;
-              while (s2 < m && off(s2 + 1) == end) { a.out[s2] = Op::init(); ++s2; }
+              while (s2 < m && off(s2 + 1) == end) { put(s2, Op::init()); ++s2; }
               s = s2;
               if (s < m) end = off(s + 1);
             }
           }
         }
       }
+    }
+  }
+  if constexpr (STAGE) {
+    if (staged) {
+      named_sync(2, TT);
+      for (int q = tid; q < out_cnt; q += TT) a.out[out_s0 + q] = stage[wpad(q)];
     }
   }
 }
@@ -1593,13 +1633,22 @@ bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n
   // a reduction's tiles write their words and leads themselves and wait for none
   if (MODE != M_REDUCE) GCVL_CK(cudaMemsetAsync(mem, 0, lookback_clear_bytes(tiles), S.stream));
   a.wmax = SEG ? wmax_for<T, MODE>(n, m) : 0;
-  bool chain = false;
-  if constexpr (MODE == M_REDUCE && SEG && std::is_same<Op, AddD>::value) {
-    chain = (long)n < RED_CHAIN_MEAN * m;
-    if (chain)
-      k_scan_tma<Op, MODE, SEG, true><<<tiles, cta_threads<MODE>(), tma_smem<T>(a.wmax), S.stream>>>(tin, tout, a);
+  bool done = false;
+  if constexpr (MODE == M_REDUCE && SEG) {
+    constexpr bool SUM = std::is_same<Op, AddD>::value;
+    if (red_staged<T>(n, m, tiles)) {
+      k_scan_tma<Op, MODE, SEG, SUM, false, true>
+          <<<tiles, cta_threads<MODE>(), tma_smem<T>(a.wmax) + TT * row_items<T>() / 32 * sizeof(T), S.stream>>>(tin, tout,
+                                                                                                             a);
+      done = true;
+    } else if constexpr (SUM) {
+      if ((long)n < RED_CHAIN_MEAN * m) {
+        k_scan_tma<Op, MODE, SEG, true><<<tiles, cta_threads<MODE>(), tma_smem<T>(a.wmax), S.stream>>>(tin, tout, a);
+        done = true;
+      }
+    }
   }
-  if (!chain) k_scan_tma<Op, MODE, SEG><<<tiles, cta_threads<MODE>(), tma_smem<T>(a.wmax), S.stream>>>(tin, tout, a);
+  if (!done) k_scan_tma<Op, MODE, SEG><<<tiles, cta_threads<MODE>(), tma_smem<T>(a.wmax), S.stream>>>(tin, tout, a);
   launch_check(name);
   if (MODE == M_REDUCE) launch_tile_fix<Op>(a.lb.word, a.lead, tiles, out);
   return true;
@@ -1875,21 +1924,23 @@ void seg_scan(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, const cha
 // (40 M elements in 1.25 M segments: 22 and 14).
 // OFFS: the CTA first scans the m <= SD_SMALL lengths itself, in shared
 // memory, and CTA 0 writes lengths and offsets: the whole descriptor in one
-// launch (vectors short enough that the grid stays within SD_SMALL_CTAS).
-constexpr int SD_BLOCK = 256, SD_RANGE = 256 * 32, SD_GRAN = SD_RANGE / kGranule;
-constexpr int SD_SMALL = 4096, SD_PER = SD_SMALL / SD_BLOCK;
+// launch (at most two ranges per SM).
+// Few ranges take 512 threads each, more than two per SM 256 (2^18 one-element
+// segments 21 us against 29; 2^25 elements in segments of 64 29 against 22).
+constexpr int SD_RANGE = 256 * 32, SD_GRAN = SD_RANGE / kGranule, SD_SMALL = 4096;
 static_assert(SD_RANGE == 32 * 256, "the bitmap is padded to whole ranges");
-template <bool OFFS>
+template <bool OFFS, int SD_BLOCK>
 __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_out, int *off, int *__restrict__ gran,
                                                      unsigned *__restrict__ bits, int n, int m) {
+  constexpr int SD_PER = SD_SMALL / SD_BLOCK;
   __shared__ unsigned s_bits[SD_RANGE / 32];
   __shared__ int s_gran[SD_GRAN];
-  __shared__ int s_first;
+  __shared__ int s_ends[2];
   __shared__ int s_off[OFFS ? SD_SMALL + SD_SMALL / 32 + 2 : 1];
   __shared__ int s_ws[SD_BLOCK / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ng = (int)(((long)n + kGranule - 1) / kGranule);
-  s_bits[tid] = 0;
+  if (tid < SD_RANGE / 32) s_bits[tid] = 0;
   if (tid < SD_GRAN) s_gran[tid] = -1;
   auto pad = [](int i) { return i + (i >> 5); };
   if constexpr (OFFS) {
@@ -1934,29 +1985,48 @@ __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_o
   auto off_at = [&](int s) { return OFFS ? s_off[pad(s)] : __ldg(off + s); };
   const long e0 = (long)blockIdx.x * SD_RANGE, e1 = min(e0 + SD_RANGE, (long)n);
   if (e0 < n) {
-    if (warp == 0) {
-      // the largest s with off[s] <= e0, 32 probes a step
-      int lo = 0, hi = m;  // off[lo] <= e0 < off[hi]
+    if (warp < 2) {
+      // the largest s with off[s] <= e, 32 probes a step: for the range's
+      // first element (warp 0) and its last (warp 1)
+      const long e = warp == 0 ? e0 : e1 - 1;
+      int lo = 0, hi = m;  // off[lo] <= e < off[hi]
       while (hi - lo > 1) {
         const int step = (hi - lo + 31) / 32, at = min(lo + lane * step, hi);
-        const unsigned below = __ballot_sync(0xffffffffu, at < hi && off_at(at) <= e0);
+        const unsigned below = __ballot_sync(0xffffffffu, at < hi && off_at(at) <= e);
         const int k = 31 - __clz(below);  // lane 0 probes lo itself
         hi = min(lo + (k + 1) * step, hi);
         lo += k * step;
       }
-      if (lane == 0) s_first = lo;
+      if (lane == 0) s_ends[warp] = lo;
     }
     __syncthreads();
-    const int first = s_first;
-    for (int s = first + tid;; s += SD_BLOCK) {
-      const int o = s < m ? off_at(s) : INT_MAX;
-      if (o >= e0 && o < e1 && off_at(s + 1) > o) {
-        const int r = (int)(o - e0);
-        atomicOr(s_bits + (r >> 5), 1u << (r & 31));
-        const int g = (r + kGranule - 1) / kGranule;
-        if (g < SD_GRAN) atomicMax(s_gran + g, s);
+    const int first = s_ends[0], last = s_ends[1];
+    for (int s0 = first + warp * 32; s0 <= last; s0 += SD_BLOCK) {
+      const int s = s0 + lane;
+      int word = -1, g = -1;
+      unsigned bit = 0;
+      if (s <= last) {
+        const int o = off_at(s);
+        if (o >= e0 && off_at(s + 1) > o) {  // a non-empty segment that starts here
+          const int r = (int)(o - e0);
+          word = r >> 5;
+          bit = 1u << (r & 31);
+          g = (r + kGranule - 1) / kGranule;
+        }
       }
-      if (!__syncthreads_or(o < e1)) break;  // offsets ascend: every thread is past the range
+      // Offsets ascend, so lanes of one word or granule are neighbours but for
+      // empty segments: the first lane of a run of equal words sets the run's
+      // bits, the last of a run of equal granules writes the largest segment
+      // (one atomic per head took six times as long on one-element segments).
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int w2 = __shfl_down_sync(0xffffffffu, word, d);
+        const unsigned b2 = __shfl_down_sync(0xffffffffu, bit, d);
+        if (lane + d < 32 && w2 == word) bit |= b2;
+      }
+      const int wprev = __shfl_up_sync(0xffffffffu, word, 1), gnext = __shfl_down_sync(0xffffffffu, g, 1);
+      if (word >= 0 && (lane == 0 || wprev != word)) atomicOr(s_bits + word, bit);
+      if (g >= 0 && g < SD_GRAN && (lane == 31 || gnext != g)) atomicMax(s_gran + g, s);
     }
     __syncthreads();
     if (tid < SD_GRAN) {
@@ -1975,7 +2045,7 @@ __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_o
       for (int w = 0; w < warp; w++) g = max(g, s_gran[32 * w + 31]);
       gran[g0 + tid] = g;
     }
-    bits[(e0 >> 5) + tid] = s_bits[tid];
+    if (tid < SD_RANGE / 32) bits[(e0 >> 5) + tid] = s_bits[tid];
   }
   if (blockIdx.x == gridDim.x - 1 && tid == 0) gran[ng] = m;
 }
@@ -1994,8 +2064,9 @@ void make_segdes(vec_p sd, vec_p l, int n, int m, vec_p scratch) {
     GCVL_CK(cudaMemsetAsync(off, 0, (size_t)((int *)bits + segdes_nbits_words(n) - off) * 4, S.stream));
     return;
   }
-  if (m <= SD_SMALL && ranges <= 2 * S.sm_count) {
-    k_segdes<true><<<ranges, SD_BLOCK, 0, S.stream>>>((const int *)l, len, off, gran, bits, n, m);
+  const bool few = ranges <= 2 * S.sm_count;
+  if (m <= SD_SMALL && few) {
+    k_segdes<true, 512><<<ranges, 512, 0, S.stream>>>((const int *)l, len, off, gran, bits, n, m);
     launch_check("mke_fov");
     return;
   }
@@ -2006,7 +2077,8 @@ void make_segdes(vec_p sd, vec_p l, int n, int m, vec_p scratch) {
   } else {
     run_scan<AddZ, M_OFFSETS, false>(off, (const int *)l, len, nullptr, m, 1, scratch, false, "mke_fov");
   }
-  k_segdes<false><<<ranges, SD_BLOCK, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
+  if (few) k_segdes<false, 512><<<ranges, 512, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
+  else k_segdes<false, 256><<<ranges, 256, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
   launch_check("mke_fov");
 }
 

@@ -231,3 +231,15 @@ def test_reduction_fix_up_by_one_cta_or_several(gpu, oracle, ranges):
     for name in ("add_red", "max_red"):
         assert np.array_equal(ops.reduce_e(gpu, name, x, lens), ops.reduce_e(oracle, name, x, lens))
     assert np.array_equal(ops.reduce_e(gpu, "add_rez", x, lens), ops.reduce_e(oracle, "add_rez", x, lens))
+
+
+@pytest.mark.parametrize("ones", [0, 1_000_000, 1_999_999])
+def test_reductions_of_nearly_one_element_segments(gpu, oracle, ones):
+    """Results put together in shared memory: one-element segments, some empty, one long at the end."""
+    r = W.rng(ones)
+    lens = np.concatenate([np.ones(ones, dtype=np.int32), r.integers(0, 3, size=2_000_000 - ones).astype(np.int32),
+                           np.array([5000, 0, 1], dtype=np.int32)])
+    n = int(lens.sum())
+    xi, xd = W.int32_uniform(r, n), r.integers(-9, 10, size=n).astype(np.float64)  # sums exact in any order
+    for name, x in (("max_rez", xi), ("add_rez", xi), ("add_red", xd), ("max_red", xd)):
+        assert np.array_equal(ops.reduce_e(gpu, name, x, lens), ops.reduce_e(oracle, name, x, lens)), name
