@@ -45,41 +45,23 @@ template <class F> void segwalk(F f, const SegView &sv, const char *name) {
   k_segwalk<F><<<grid_for(((long)sv.n + SITEMS - 1) / SITEMS, VBLOCK), VBLOCK, 0, stream()>>>(f, sv);
   launch_check(name);
 }
-// Segmented maps whose result is one value per element (DIST, INDEX,
-// segmented BPERMUTE): a warp owns SMI*32 consecutive elements, each lane
-// SMI consecutive ones.  Phase 1 walks the lane's elements through the
-// segment descriptor (one segment lookup, then a walk) and records a token
-// per element (the segment, or the source address); phase 2 fetches all
-// the lane's values at once (independent loads in flight); the values pass
-// through shared memory so that every global load and store is coalesced.
-#ifndef GCVL_SMI
-#define GCVL_SMI 16
-#endif
-#ifndef GCVL_SMB
-#define GCVL_SMB 128
-#endif
-constexpr int SMI = GCVL_SMI, SMB = GCVL_SMB;
-template <class F>
+// Segmented maps whose result is one value per element (DIST, INDEX): a warp
+// owns SMI*32 consecutive elements, each lane SMI consecutive ones.  A lane
+// walks its elements through the segment descriptor (one segment lookup, then
+// a walk) and fetches each one's value; the values pass through shared memory
+// so that every global store is coalesced.
+constexpr int SMB = 128;  // threads per CTA (256: up to 15 % slower)
+template <class F, int SMI>
 __global__ void __launch_bounds__(SMB) k_segmap(F f, SegView sv) {
   typedef typename F::T T;
   constexpr int WE = 32 * SMI, PADW = WE + 32;
   __shared__ T s_val[SMB / 32][PADW];
-  __shared__ int s_aux[F::AUX ? SMB / 32 : 1][F::AUX ? PADW : 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long wbase = ((long)blockIdx.x * (SMB / 32) + warp) * WE;
   if (wbase >= sv.n) return;
   const int wcnt = (int)min((long)WE, (long)sv.n - wbase);
-  if constexpr (F::AUX) {
-#pragma unroll
-    for (int j = 0; j < SMI; j++) {
-      const int e = j * 32 + lane;
-      if (e < wcnt) s_aux[warp][e + e / SMI] = __ldcs(f.aux + wbase + e);
-    }
-    __syncwarp();
-  }
   const int e0 = lane * SMI;
   const int cnt = max(0, min(SMI, wcnt - e0));
-  long long tok[SMI];
   if (cnt > 0) {
     const int k0 = (int)(wbase + e0);
     int sg = seg_of(sv, k0);
@@ -89,22 +71,9 @@ __global__ void __launch_bounds__(SMB) k_segmap(F f, SegView sv) {
       if (i < cnt) {
         const int k = k0 + i;
         while (k >= end) { ++sg; start = end; end = __ldg(sv.off + sg + 1); }
-        int a = 0;
-        if constexpr (F::AUX) a = s_aux[warp][e0 + lane + i];
-        tok[i] = f.token(k, sg, start, a);
-        // values that come from a per-segment table are fetched in the walk
-        if constexpr (!F::GATHER) s_val[warp][e0 + lane + i] = f.fetch(tok[i]);
+        s_val[warp][e0 + lane + i] = f(k, sg, start);
       }
     }
-  }
-  if constexpr (F::GATHER) {  // all of the lane's gathers in flight at once
-    T v[SMI];
-#pragma unroll
-    for (int i = 0; i < SMI; i++)
-      if (i < cnt) v[i] = f.fetch(tok[i]);
-#pragma unroll
-    for (int i = 0; i < SMI; i++)
-      if (i < cnt) s_val[warp][e0 + lane + i] = v[i];
   }
   __syncwarp();
 #pragma unroll
@@ -113,10 +82,13 @@ __global__ void __launch_bounds__(SMB) k_segmap(F f, SegView sv) {
     if (e < wcnt) __stcs(f.d + wbase + e, s_val[warp][e + e / SMI]);
   }
 }
+// A lane walks 16 elements, 8 where segments average under 4: the walk's loads
+// follow one another, one per segment (DIST at 2^25, 16 / 8, us: mean 1 177 /
+// 104, 1.5 115 / 74, 3 62 / 62, 8 43 / 46, 64 32 / 35).
 template <class F> void segmap(F f, const SegView &sv, const char *name) {
   if (sv.n <= 0 || sv.m <= 0) return;
-  const long per = (long)SMB * SMI;
-  k_segmap<F><<<(int)((sv.n + per - 1) / per), SMB, 0, stream()>>>(f, sv);
+  if ((long)sv.n < 4L * sv.m) k_segmap<F, 8><<<ceil_div(sv.n, SMB * 8), SMB, 0, stream()>>>(f, sv);
+  else k_segmap<F, 16><<<ceil_div(sv.n, SMB * 16), SMB, 0, stream()>>>(f, sv);
   launch_check(name);
 }
 // Segmented permute, d[start(seg(k)) + i[k]] = s[k]: a warp owns SMI*32
@@ -124,6 +96,15 @@ template <class F> void segmap(F f, const SegView &sv, const char *name) {
 // segment descriptor and records their segment starts in shared memory;
 // then the index and value loads are coalesced (element j*32 + lane) and
 // all of a lane's stores are in flight together.
+// Elements a lane walks in the segmented permutes: at 2^25 in segments of 64,
+// 16 / 8 / 6 / 4 elements, us: smp_pez 94 / 86 / 89 / 88, smp_ped 126 / 112 /
+// 107 / 109, bck_pez 98 / 81 / 74 / 85, bck_ped 121 / 115 / 109 / 109; in
+// one-element segments 140 / 117 / 114 / 114, 189 / 154 / 138 / 144, 183 /
+// 127 / 101 / 120, 195 / 156 / 140 / 141.
+#ifndef GCVL_SMI
+#define GCVL_SMI 6
+#endif
+constexpr int SMI = GCVL_SMI;
 template <class T>
 __global__ void __launch_bounds__(SMB) k_segscatter(T *__restrict__ d, const T *__restrict__ s,
                                                     const int *__restrict__ idx, SegView sv) {
@@ -169,28 +150,79 @@ template <class T> void segscatter(T *d, const T *s, const int *idx, const SegVi
   launch_check(name);
 }
 
+// Segmented back-permute with as many source as destination segments,
+// d[k] = s[off_s[seg(k)] + i[k]]: the same walk, which records each element's
+// source segment start; the index loads go out before it, and a lane then
+// gathers for elements 32 apart, so that one load of the warp reads the
+// sources of 32 neighbours -- mostly one segment -- and not those of 32
+// elements 16 apart, whose loads hit a line each and whose results then went
+// through shared memory (2^25 elements in segments of 64: bck_ped 233 -> 109
+// us, its bytes take 100; bck_pez 102 -> 74, 60).
+template <class T>
+__global__ void __launch_bounds__(SMB) k_seggather(T *__restrict__ d, const T *__restrict__ s,
+                                                   const int *__restrict__ idx, const int *__restrict__ off_s,
+                                                   SegView sv) {
+  constexpr int WE = 32 * SMI, PADW = WE + 32;
+  __shared__ int s_start[SMB / 32][PADW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long wbase = ((long)blockIdx.x * (SMB / 32) + warp) * WE;
+  if (wbase >= sv.n) return;
+  const int wcnt = (int)min((long)WE, (long)sv.n - wbase);
+  int ix[SMI];
+#pragma unroll
+  for (int j = 0; j < SMI; j++) {
+    const int e = j * 32 + lane;
+    if (e < wcnt) ix[j] = __ldcs(idx + wbase + e);
+  }
+  const int e0 = lane * SMI;
+  const int cnt = max(0, min(SMI, wcnt - e0));
+  if (cnt > 0) {
+    const int k0 = (int)(wbase + e0);
+    int sg = seg_of(sv, k0);
+    int end = __ldg(sv.off + sg + 1), start = __ldg(off_s + sg);
+#pragma unroll
+    for (int i = 0; i < SMI; i++) {
+      if (i < cnt) {
+        if (k0 + i >= end) {
+          do { ++sg; end = __ldg(sv.off + sg + 1); } while (k0 + i >= end);
+          start = __ldg(off_s + sg);
+        }
+        s_start[warp][e0 + lane + i] = start;  // element e at e + e / SMI
+      }
+    }
+  }
+  __syncwarp();
+  T v[SMI];
+#pragma unroll
+  for (int j = 0; j < SMI; j++) {
+    const int e = j * 32 + lane;
+    if (e < wcnt) v[j] = __ldg(s + (long)s_start[warp][e + e / SMI] + ix[j]);
+  }
+#pragma unroll
+  for (int j = 0; j < SMI; j++) {
+    const int e = j * 32 + lane;
+    if (e < wcnt) __stcs(d + wbase + e, v[j]);
+  }
+}
+template <class T>
+void seggather(T *d, const T *s, const int *idx, const int *off_s, const SegView &sv, const char *name) {
+  if (sv.n <= 0 || sv.m <= 0) return;
+  const long per = (long)SMB * SMI;
+  k_seggather<T><<<(int)((sv.n + per - 1) / per), SMB, 0, stream()>>>(d, s, idx, off_s, sv);
+  launch_check(name);
+}
+
 template <class TT> struct DisMap {  // d[k] = v[seg(k)]
   typedef TT T;
-  static constexpr bool AUX = false, GATHER = false;
-  T *d; const T *v; const int *aux;
-  __device__ long long token(int, int s, int, int) const { return s; }
-  __device__ T fetch(long long s) const { return __ldg(v + s); }
+  T *d; const T *v;
+  __device__ T operator()(int, int s, int) const { return __ldg(v + s); }
 };
 struct IndMap {  // d[k] = init[s] + stride[s] * (k - start)
   typedef int T;
-  static constexpr bool AUX = false, GATHER = false;
-  int *d; const int *init; const int *stride; const int *aux;
-  __device__ long long token(int k, int s, int start, int) const {
+  int *d; const int *init; const int *stride;
+  __device__ int operator()(int k, int s, int start) const {
     return (int)((unsigned)__ldg(init + s) + (unsigned)__ldg(stride + s) * (unsigned)(k - start));
   }
-  __device__ int fetch(long long v) const { return (int)v; }
-};
-template <class TT> struct BPermMap {  // d[k] = s[off_s[seg_d(k)] + i[k]], as many source as dest segments
-  typedef TT T;
-  static constexpr bool AUX = true, GATHER = true;
-  T *d; const T *src; const int *off_s; const int *aux;
-  __device__ long long token(int, int s, int, int i) const { return (long long)__ldg(off_s + s) + i; }
-  __device__ T fetch(long long at) const { return __ldg(src + at); }
 };
 
 // f(i) for i in [0, n)
@@ -842,7 +874,7 @@ using namespace gcvl;
   META_SEG(rep_ve##L, INPLACE_NONE)                                                    \
   GCVL_EXPORT void dis_ve##L(vec_p d, vec_p v, vec_p sd, int n, int m, vec_p scratch) { \
     (void)scratch; ensure_init();                                                     \
-    segmap(DisMap<T>{(T *)d, (const T *)v, nullptr}, seg_view(sd, n, m), "dis_ve" #L); \
+    segmap(DisMap<T>{(T *)d, (const T *)v}, seg_view(sd, n, m), "dis_ve" #L); \
   }                                                                                    \
   META_SEG(dis_ve##L, INPLACE_NONE)
 EXT_REP(z, int)
@@ -873,7 +905,7 @@ META1(rep_vud, INPLACE_NONE)
 // Segmented index (library.c:28-49).
 GCVL_EXPORT void ind_lez(vec_p d, vec_p init, vec_p stride, vec_p sd, int n, int m, vec_p scratch) {
   (void)scratch; ensure_init();
-  segmap(IndMap{(int *)d, (const int *)init, (const int *)stride, nullptr}, seg_view(sd, n, m), "ind_lez");
+  segmap(IndMap{(int *)d, (const int *)init, (const int *)stride}, seg_view(sd, n, m), "ind_lez");
 }
 META_SEG(ind_lez, INPLACE_NONE)
 
@@ -906,8 +938,7 @@ META_SEG(ind_lez, INPLACE_NONE)
     if (m_s == 1) { gather_src<T>((T *)d, (const T *)s, (const int *)i, n_d, n_s, scratch, "bck_pe" #L); return; } \
     SegView ss = seg_view(sd_s, n_s, m_s);                                              \
     if (m_s == m_d)                                                                     \
-      segmap(BPermMap<T>{(T *)d, (const T *)s, ss.off, (const int *)i},                  \
-             seg_view(sd_d, n_d, m_d), "bck_pe" #L);                                    \
+      seggather<T>((T *)d, (const T *)s, (const int *)i, ss.off, seg_view(sd_d, n_d, m_d), "bck_pe" #L); \
     else                                                                                \
       segwalk(BPermSeg<T>{(T *)d, (const T *)s, (const int *)i, ss.off, m_s},               \
               seg_view(sd_d, n_d, m_d), "bck_pe" #L);                                   \

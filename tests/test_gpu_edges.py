@@ -243,3 +243,23 @@ def test_reductions_of_nearly_one_element_segments(gpu, oracle, ones):
     xi, xd = W.int32_uniform(r, n), r.integers(-9, 10, size=n).astype(np.float64)  # sums exact in any order
     for name, x in (("max_rez", xi), ("add_rez", xi), ("add_red", xd), ("max_red", xd)):
         assert np.array_equal(ops.reduce_e(gpu, name, x, lens), ops.reduce_e(oracle, name, x, lens)), name
+
+
+@pytest.mark.parametrize("n", [1, 31, 191, 192, 193, 767, 768, 769, 20_003])
+@pytest.mark.parametrize("shape", ["one-element", "long", "geometric"])
+@pytest.mark.parametrize("t", "zbd")
+def test_segmented_permutes_at_warp_edges(gpu, oracle, t, shape, n):
+    """A warp takes 192 elements (32 lanes of 6), a CTA 768."""
+    r = W.rng(n + ord(t))
+    lens = _lens(r, n, shape)
+    x = _keys(r, n, t, "few" if t == "b" else "uniform")
+    perm = W.seg_permutation(r, lens)
+    len_s = (lens + r.integers(0, 4, size=lens.size)).astype(np.int32)  # as many source segments
+    xs = _keys(r, int(len_s.sum()), t, "few" if t == "b" else "uniform")
+    idx = W.seg_indices(r, len_s, lens)
+    v, ii = _keys(r, lens.size, t, "few" if t == "b" else "uniform"), W.int32_uniform(r, lens.size)
+    for R in (gpu, oracle):
+        R.got = [ops.smp_e(R, f"smp_pe{t}", x, perm, lens), ops.bck_e(R, f"bck_pe{t}", xs, idx, len_s, lens),
+                 ops.dis_e(R, f"dis_ve{t}", v, lens), ops.ind_e(R, ii, ii[::-1].copy(), lens)]
+    for a, b in zip(gpu.got, oracle.got):
+        assert np.array_equal(a, b)
