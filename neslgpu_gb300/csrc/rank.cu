@@ -65,16 +65,12 @@ constexpr int RK_MAXPASS = 12;
 #ifndef GCVL_RK_MINB_NARROW
 #define GCVL_RK_MINB_NARROW 3
 #endif
-// Vectors of at most 2^20 elements take smaller tiles, so that more CTAs work
-// (int / double ranks: 2^20 keys in tiles of 20 items 95 / 176 us, 16 items
-// 79 / 150, 8 items 88 / 173; 2^18 keys 67 / 117, 59 / 102, 55 / 100; at 2^21
-// 20 items win again, 108 / 244 against 121 / 232).
-#ifndef GCVL_RK_ITEMS_SMALL
-#define GCVL_RK_ITEMS_SMALL 16
-#endif
-constexpr int RK_ITEMS_SMALL = GCVL_RK_ITEMS_SMALL, RK_SMALL_MAX = 1 << 20;
+// Shorter vectors take smaller tiles, so that more CTAs work.  Int / double
+// ranks in tiles of 20, 16 and 8 items a thread, us: 2^21 keys 108 / 244, 121 /
+// 232; 2^20 95 / 176, 79 / 150, 88 / 173; 2^18 67 / 117, 59 / 102, 55 / 100;
+// 2^13 50 / 91, 41 / 78, 33 / 60.
+constexpr int RK_ITEMS_SMALL = 16, RK_SMALL_MAX = 1 << 20, RK_ITEMS_TINY = 8, RK_TINY_MAX = 1 << 18;
 constexpr int RK_LB = GCVL_RK_LB;  // predecessors read per look-back round trip
-static_assert(RK_ITEMS_SMALL != RK_ITEMS_LARGE, "the tile tells the two forms apart");
 constexpr int RK_DIRECT_MAX = 1 << 23;
 // 8 measured best at 2^28 (bck_puz / smp_puz): 4 items 2.87 / 2.94 ms,
 // 8 items 2.63 / 2.78, 16 items 3.01 / 2.78
@@ -806,11 +802,15 @@ void launch_pass_items(const PassArgs<K, V> &a) {
   k_radix_pass<K, V, AUX, IN, OUT, ITEMS, DYN><<<grid, RK_BLOCK, sm, stream()>>>(a);
   launch_check("k_radix_pass");
 }
-inline bool rk_small(long n) { return n <= RK_SMALL_MAX; }
-inline int rk_tile(long n) { return RK_BLOCK * (rk_small(n) ? RK_ITEMS_SMALL : RK_ITEMS_LARGE); }
+inline int rk_tile(long n) {
+  return RK_BLOCK * (n <= RK_TINY_MAX ? RK_ITEMS_TINY : n <= RK_SMALL_MAX ? RK_ITEMS_SMALL : RK_ITEMS_LARGE);
+}
 template <class K, class V, bool AUX, int IN, int OUT, bool DYN> void launch_pass(const PassArgs<K, V> &a) {
-  if (!rk_small(a.n)) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_LARGE, DYN>(a);
-  else if constexpr (OUT != OUT_WIN) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_SMALL, DYN>(a);
+  if (a.n > RK_SMALL_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_LARGE, DYN>(a);
+  else if constexpr (OUT != OUT_WIN) {
+    if (a.n > RK_TINY_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_SMALL, DYN>(a);
+    else launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_TINY, DYN>(a);
+  }
 }
 static_assert(RK_SMALL_MAX <= RK_DIRECT_MAX, "windows only for large tiles");
 
@@ -1103,7 +1103,9 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
                                                        state[0], (long)(state_bytes / 4), rk_tile(n));
     launch_check("k_rank_prep_long");
   } else {
-    const int pg = std::min(S.sm_count * 8, ceil_div(n, (long)RK_BLOCK));
+    // at least 16 keys a thread: every CTA adds its histograms to the vector's
+    // with an atomic per bin (2^20 keys by 1216 CTAs 14.6 us, by 256 5)
+    const int pg = std::min(S.sm_count * 8, ceil_div(n, (long)RK_BLOCK * 16));
     k_rank_prep<K><<<pg, RK_BLOCK, 0, S.stream>>>((const K *)s, n, up, hist, (uint4 *)state[0],
                                                   (long)(3 * state_bytes / 16));
     launch_check("k_rank_prep");

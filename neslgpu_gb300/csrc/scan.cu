@@ -1522,6 +1522,18 @@ template <class T> constexpr size_t tma_smem(int wmax) {
   return 1024 + (size_t)TT * row_items<T>() * sizeof(T) + (size_t)(wmax > 0 ? wpad(wmax) + 1 : 0) * 4;
 }
 
+// Scans of at most this many elements take k_scan, one tile per CTA: while the
+// tiles are few, the ring's two rounds and its load by TMA only add latency.
+// k_scan / ring, us: add_sez 2^14 6.2 / 8.3, 2^18 6.3 / 8.6, 2^20 10.2 / 12.3,
+// 2^22 14.4 / 16.4, 2^23 22.5 / 18.4; add_suz 2^21 15.3 / 17.0, 2^22 22.3 /
+// 20.5; add_sed 2^14 8.9 / 11.4, 2^18 9.2 / 15.4, 2^19 13.3 / 16.4, 2^20 20.5 /
+// 18.7; max_sed 2^18 10.2 / 17.2, 2^21 30.7 / 42.1, 2^22 50.3 / 51.3, 2^24 166 / 156;
+// mul_sed 2^21 28.7 / 34.5, 2^22 47.4 / 43.0.  Float64 + is added in FP64 there,
+// not in fixed point: the error against exact sums is the smaller of the two.
+template <class Op, bool SEG> constexpr long ring_above() {
+  if (std::is_same<Op, AddD>::value) return 1L << 19;
+  return SEG && !std::is_same<Op, MulD>::value ? 1L << 22 : 1L << 21;
+}
 // CTAs of a ring scan: as many as are resident at once (0: it does not fit)
 template <class Op, bool SEG> int ring_grid(int tiles) {
   static int per_sm = -1;
@@ -1568,6 +1580,7 @@ bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n
   CUtensorMap tin, tout;
   State &S = st();
   if constexpr (MODE == M_SCAN) {
+    if (n <= ring_above<Op, SEG>()) return false;
     const int tiles = ceil_div(n, (long)RTT * row_items<T>());
     const int grid = ring_grid<Op, SEG>(tiles);
     if (grid > 0) {

@@ -26,7 +26,7 @@ def test_rand_group_edges(gpu, oracle, n):
 # ----------------------------------------------------------------- ranks ---
 # sizes of neslgpu_gb300/csrc/rank.cuh and rank.cu: a CTA's segments start in
 # 2048 elements and hold at most 2048; one CTA ranks a whole vector of 4096;
-# digit passes take small tiles up to 2^20 and write ranks by window past 2^23
+# digit passes take smaller tiles up to 2^18 and up to 2^20 and write ranks by window past 2^23
 LR_T = LR_MAX = 2048
 
 
@@ -74,7 +74,7 @@ def test_rank_segments(gpu, oracle, name, dist, shape):
     assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 2047, 2049, 4095, 4096, 4097, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 257, 2047, 2049, 4095, 4096, 4097, 1 << 18, (1 << 18) + 1, 1 << 20, (1 << 20) + 1])
 @pytest.mark.parametrize("name,dist", [("rku_luz", "uniform"), ("rkd_luz", "few"), ("rku_lud", "special"),
                                        ("rkd_lud", "uniform"), ("rku_luz", "clusters")])
 def test_rank_whole_vectors(gpu, oracle, name, dist, n):
@@ -263,3 +263,32 @@ def test_segmented_permutes_at_warp_edges(gpu, oracle, t, shape, n):
                  ops.dis_e(R, f"dis_ve{t}", v, lens), ops.ind_e(R, ii, ii[::-1].copy(), lens)]
     for a, b in zip(gpu.got, oracle.got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("name,n", [("add_sez", 1 << 22), ("add_sez", (1 << 22) + 1), ("max_sed", 1 << 22),
+                                    ("max_sed", (1 << 22) + 1), ("add_suz", 1 << 21), ("add_suz", (1 << 21) + 1),
+                                    ("min_sud", (1 << 21) + 1)])
+def test_scans_either_side_of_the_ring(gpu, oracle, name, n):
+    r = W.rng(n)
+    x = _keys(r, n, name[-1], "uniform")
+    if name[5] == "u":
+        assert np.array_equal(ops.scan_u(gpu, name, x), ops.scan_u(oracle, name, x))
+    else:
+        lens = W.with_empty(r, W.lognormal_lengths(r, n, 5, 2, 1 << 20), 0.1)
+        assert np.array_equal(ops.scan_e(gpu, name, x, lens), ops.scan_e(oracle, name, x, lens))
+
+
+@pytest.mark.parametrize("n", [1 << 19, (1 << 19) + 1])
+@pytest.mark.parametrize("name", ["add_sed", "add_sud"])
+def test_float_sums_either_side_of_the_ring(gpu, oracle, name, n):
+    """Within 1e-12 of the magnitudes summed, as for every float64 sum."""
+    r = W.rng(n + 5)
+    x = W.float64_normal(r, n) * 2.0 ** r.integers(-40, 40, size=n)
+    lens = W.lognormal_lengths(r, n, 5, 2, 1 << 18) if name == "add_sed" else np.array([n], dtype=np.int32)
+    c = np.concatenate([[0.0], np.cumsum(np.abs(x))])
+    mag = c[np.arange(n)] - np.repeat(c[np.cumsum(lens) - lens], lens)
+    if name == "add_sed":
+        g, o = ops.scan_e(gpu, name, x, lens), ops.scan_e(oracle, name, x, lens)
+    else:
+        g, o = ops.scan_u(gpu, name, x), ops.scan_u(oracle, name, x)
+    assert np.all(np.abs(g - o) <= 1e-12 * np.maximum(mag, np.abs(o)))
