@@ -103,6 +103,7 @@ class Ins:
     a: object = None   # COPY/POP/CPOP count; CALL target name; CONST value
     b: object = None   # COPY/POP/CPOP depth; branch target
     line: int = 0
+    x: object = None   # the interpreter's: the library functions the instruction calls, once looked up
 
 
 _TOKEN = re.compile(r"\{[^}]*\}|\(|\)|\"[^\"]*\"|[^\s(){}\"]+")
@@ -229,7 +230,7 @@ class Heap:
 
     def __init__(self, c: CVL):
         self.c = c
-        self.free: dict[int, list[int]] = {}
+        self.free: dict[int, list[int]] = {}  # negated addresses, ascending: the last entry is the lowest address
         self.held = 0
         self.no_new = False
         self.on_trim = None  # called when blocks go back to the device
@@ -242,12 +243,16 @@ class Heap:
 
     def alloc(self, units: int) -> tuple[int, int]:
         cls = self.size_class(units)
+        return self.take(cls), cls
+
+    def take(self, cls: int) -> int:
+        """A block of the size class."""
         lst = self.free.get(cls)
         if lst:
-            p = lst.pop()
+            p = -lst.pop()
             if self.log is not None:
                 self.log.append(("a", cls, p))
-            return p, cls
+            return p
         if self.no_new:  # a captured or replayed block may not allocate
             raise _NeedsHost("heap")
         p = self.c.alo_foz(cls)
@@ -257,15 +262,17 @@ class Heap:
             if not p:
                 raise MemoryError(f"alo_foz({cls}) failed")
         self.held += cls
-        return p, cls
+        return p
 
     def release(self, ptr: int, cls: int):
-        # each class's free list is kept in descending address order and
-        # allocation takes the lowest address: which addresses a sequence of
+        # allocation takes a class's lowest address: which addresses a sequence of
         # requests gets then depends only on which blocks are free, not on
         # the order they were freed in, so a block that runs again in the same
         # state gets the same vectors (graph replay relies on it)
-        bisect.insort(self.free.setdefault(cls, []), ptr, key=lambda q: -q)
+        lst = self.free.get(cls)
+        if lst is None:
+            lst = self.free[cls] = []
+        bisect.insort(lst, -ptr)
         if self.log is not None:
             self.log.append(("r", cls, ptr))
 
@@ -274,7 +281,7 @@ class Heap:
             self.on_trim()
         for cls, lst in self.free.items():
             for p in lst:
-                self.c.fre_fov(p)
+                self.c.fre_fov(-p)
                 self.held -= cls
         self.free.clear()
 
@@ -411,6 +418,8 @@ class Interpreter:
         self.timer = 0.0
         self.ops_run = 0
         self._fn = {}
+        self._sizes: dict = {}    # (kind, length, elements of a descriptor) -> size class
+        self._scr_units: dict = {}  # (id of F_scratch, its arguments) -> units
         # VCODE file descriptors: 0, 1, 2 are the standard streams
         self.files: dict[int, _VStream] = {0: _VStream(sys.stdin), 1: _VStream(sys.stdout), 2: _VStream(sys.stderr)}
         # trace(op, typ, consumed, produced): called after every vector
@@ -442,9 +451,36 @@ class Interpreter:
             return c.siz_fod(max(length, 1))
         return c.siz_foz(max(length, 1)) if kind == "I" else c.siz_fob(max(length, 1))
 
+    # F_scratch and the sizes depend on their arguments alone, and programs ask
+    # for the same ones over and over: the answers are kept (at most
+    # _KEEP_SIZES of them, then none)
+    _KEEP_SIZES = 1 << 14
+
     def new(self, kind, length, seg_len=None) -> Vec:
-        ptr, cls = self.heap.alloc(self.units(kind, length, seg_len))
-        return Vec(kind, length, seg_len if kind == "S" else None, ptr, cls)
+        if kind != "S":
+            seg_len = None
+        key = (kind, length, seg_len)
+        cls = self._sizes.get(key)
+        if cls is None:
+            if len(self._sizes) >= self._KEEP_SIZES:
+                self._sizes.clear()
+            cls = self._sizes[key] = Heap.size_class(self.units(kind, length, seg_len))
+        return Vec(kind, length, seg_len, self.heap.take(cls), cls)
+
+    def bind(self, ins, name):
+        """The function `name` and its F_scratch, kept with the instruction."""
+        ins.x = (self.fn(name), self.sfn(name + "_scratch"))
+        return ins.x
+
+    def scratch_for(self, sfn, *sizes):
+        """The scratch vector of a call, sized by its F_scratch."""
+        key = (id(sfn), sizes)  # sfn is one of self._fn, which keeps it
+        u = self._scr_units.get(key)
+        if u is None:
+            if len(self._scr_units) >= self._KEEP_SIZES:
+                self._scr_units.clear()
+            u = self._scr_units[key] = sfn(*sizes)
+        return self.scratch(u) if u > self.scratch_units else self.scratch_ptr
 
     def drop(self, v: Vec):
         v.ref -= 1
@@ -541,9 +577,9 @@ class Interpreter:
     def segdes_from_lengths(self, lens: Vec) -> Vec:
         c = self.c
         m = lens.len
-        n = int(self.fn("add_ruz")(lens.ptr, m, self.scratch(self.sfn("add_ruz_scratch")(m)))) if m else 0
+        n = int(self.fn("add_ruz")(lens.ptr, m, self.scratch_for(self.sfn("add_ruz_scratch"), m))) if m else 0
         sd = self.new("S", m, n)
-        self.fn("mke_fov")(sd.ptr, lens.ptr, n, m, self.scratch(self.sfn("mke_fov_scratch")(n, m)))
+        self.fn("mke_fov")(sd.ptr, lens.ptr, n, m, self.scratch_for(self.sfn("mke_fov_scratch"), n, m))
         return sd
 
     # -- main loop
@@ -569,18 +605,29 @@ class Interpreter:
             self.ops_run += 1
             if op == "COPY":
                 k, d = ins.a, ins.b
+                if k == 1:
+                    v = st[-1 - d]
+                    v.ref += 1
+                    st.append(v)
+                    continue
                 seg = st[len(st) - d - k: len(st) - d]
                 for v in seg:
                     v.ref += 1
                 st.extend(seg)
             elif op == "CPOP":
                 k, d = ins.a, ins.b
+                if k == 1:
+                    st.append(st.pop(-1 - d))
+                    continue
                 lo, hi = len(st) - d - k, len(st) - d
                 seg = st[lo:hi]
                 del st[lo:hi]
                 st.extend(seg)
             elif op == "POP":
                 k, d = ins.a, ins.b
+                if k == 1:
+                    self.drop(st.pop(-1 - d))
+                    continue
                 lo, hi = len(st) - d - k, len(st) - d
                 for v in st[lo:hi]:
                     self.drop(v)
@@ -645,18 +692,29 @@ class Interpreter:
             self.ops_run += 1
             if op == "COPY":
                 k, d = ins.a, ins.b
+                if k == 1:
+                    v = st[-1 - d]
+                    v.ref += 1
+                    st.append(v)
+                    continue
                 seg = st[len(st) - d - k: len(st) - d]
                 for v in seg:
                     v.ref += 1
                 st.extend(seg)
             elif op == "CPOP":
                 k, d = ins.a, ins.b
+                if k == 1:
+                    st.append(st.pop(-1 - d))
+                    continue
                 lo, hi = len(st) - d - k, len(st) - d
                 seg = st[lo:hi]
                 del st[lo:hi]
                 st.extend(seg)
             elif op == "POP":
                 k, d = ins.a, ins.b
+                if k == 1:
+                    self.drop(st.pop(-1 - d))
+                    continue
                 lo, hi = len(st) - d - k, len(st) - d
                 for v in st[lo:hi]:
                     self.drop(v)
@@ -726,7 +784,7 @@ class Interpreter:
             if op == "a":
                 free[c].pop()
             else:
-                bisect.insort(free.setdefault(c, []), ptr, key=lambda q: -q)
+                bisect.insort(free.setdefault(c, []), -ptr)
         st[base:] = [top[j] if w == "o" else (news[j] if w == "n" else j) for w, j in rec["out"]]
         self.ops_run += end - pc
         if self.c.gcvl_graph_launch(rec["graph"]) != 0:
@@ -907,28 +965,26 @@ class Interpreter:
         op, st = ins.op, self.stack
         if op in ELT:
             stem, ar, res = ELT[op]
-            t = ins.typ or ELT_DEFAULT_TYPE.get(op) or "INT"
+            fn, sfn = ins.x or self.bind(ins, f"{stem}_wu{TYPE_SUFFIX[ins.typ or ELT_DEFAULT_TYPE.get(op) or 'INT']}")
             args = st[-ar:]
             a0 = args[0]
             kind = a0.kind if res is None else (args[1].kind if res == "A2" else res)
             L = a0.seg_len if a0.kind == "S" else a0.len
             d = self.new(kind, L)
-            name = f"{stem}_wu{TYPE_SUFFIX[t]}"
-            scr = self.scratch(self.sfn(name + "_scratch")(L))
-            self.fn(name)(d.ptr, *[a.ptr for a in args], L, scr)
+            fn(d.ptr, *[a.ptr for a in args], L, self.scratch_for(sfn, L))
             self._finish(ar, [d])
         elif op in SCAN or op in REDUCE or op in ("RANK_UP", "RANK_DOWN"):
-            t = TYPE_SUFFIX[ins.typ or "INT"]
             x, sd = st[-2], st[-1]
             if op in SCAN:
-                name, kind, L = f"{SCAN[op]}_se{t}", x.kind, x.len
+                fs = ins.x or self.bind(ins, f"{SCAN[op]}_se{TYPE_SUFFIX[ins.typ or 'INT']}")
+                d = self.new(x.kind, x.len)
             elif op in REDUCE:
-                name, kind, L = f"{REDUCE[op]}_re{t}", x.kind, sd.len
+                fs = ins.x or self.bind(ins, f"{REDUCE[op]}_re{TYPE_SUFFIX[ins.typ or 'INT']}")
+                d = self.new(x.kind, sd.len)
             else:
-                name, kind, L = ("rku_le" if op == "RANK_UP" else "rkd_le") + t, "I", x.len
-            d = self.new(kind, L)
-            scr = self.scratch(self.sfn(name + "_scratch")(sd.seg_len, sd.len))
-            self.fn(name)(d.ptr, x.ptr, sd.ptr, sd.seg_len, sd.len, scr)
+                fs = ins.x or self.bind(ins, ("rku_le" if op == "RANK_UP" else "rkd_le") + TYPE_SUFFIX[ins.typ or "INT"])
+                d = self.new("I", x.len)
+            fs[0](d.ptr, x.ptr, sd.ptr, sd.seg_len, sd.len, self.scratch_for(fs[1], sd.seg_len, sd.len))
             self._finish(2, [d])
         elif op == "MAKE_SEGDES":
             lens = st[-1]
@@ -937,8 +993,8 @@ class Interpreter:
         elif op == "LENGTHS":
             sd = st[-1]
             d = self.new("I", sd.len)
-            self.fn("len_fos")(d.ptr, sd.ptr, sd.seg_len, sd.len,
-                               self.scratch(self.sfn("len_fos_scratch")(sd.seg_len, sd.len)))
+            fn, sfn = ins.x or self.bind(ins, "len_fos")
+            fn(d.ptr, sd.ptr, sd.seg_len, sd.len, self.scratch_for(sfn, sd.seg_len, sd.len))
             self._finish(1, [d])
         elif op == "LENGTH":
             v = st[-1]
@@ -946,26 +1002,22 @@ class Interpreter:
         elif op == "PACK":
             self._pack(ins)
         elif op == "DIST":
-            t = TYPE_SUFFIX[ins.typ or "INT"]
+            fn, sfn = ins.x or self.bind(ins, "dis_ve" + TYPE_SUFFIX[ins.typ or "INT"])
             v, sd = st[-2], st[-1]
             d = self.new(v.kind, sd.seg_len)
-            name = f"dis_ve{t}"
-            self.fn(name)(d.ptr, v.ptr, sd.ptr, sd.seg_len, sd.len,
-                          self.scratch(self.sfn(name + "_scratch")(sd.seg_len, sd.len)))
+            fn(d.ptr, v.ptr, sd.ptr, sd.seg_len, sd.len, self.scratch_for(sfn, sd.seg_len, sd.len))
             self._finish(2, [d])
         elif op == "INDEX":
             init, stride, sd = st[-3], st[-2], st[-1]
             d = self.new("I", sd.seg_len)
-            self.fn("ind_lez")(d.ptr, init.ptr, stride.ptr, sd.ptr, sd.seg_len, sd.len,
-                               self.scratch(self.sfn("ind_lez_scratch")(sd.seg_len, sd.len)))
+            fn, sfn = ins.x or self.bind(ins, "ind_lez")
+            fn(d.ptr, init.ptr, stride.ptr, sd.ptr, sd.seg_len, sd.len, self.scratch_for(sfn, sd.seg_len, sd.len))
             self._finish(3, [d])
         elif op == "EXTRACT":
-            t = TYPE_SUFFIX[ins.typ or "INT"]
+            fn, sfn = ins.x or self.bind(ins, "ext_ve" + TYPE_SUFFIX[ins.typ or "INT"])
             x, idx, sd = st[-3], st[-2], st[-1]
             d = self.new(x.kind, idx.len)
-            name = f"ext_ve{t}"
-            self.fn(name)(d.ptr, x.ptr, idx.ptr, sd.ptr, sd.seg_len, sd.len,
-                          self.scratch(self.sfn(name + "_scratch")(sd.seg_len, sd.len)))
+            fn(d.ptr, x.ptr, idx.ptr, sd.ptr, sd.seg_len, sd.len, self.scratch_for(sfn, sd.seg_len, sd.len))
             self._finish(3, [d])
         elif op == "REPLACE":
             t = TYPE_SUFFIX[ins.typ or "INT"]
@@ -982,33 +1034,28 @@ class Interpreter:
                           self.scratch(self.sfn(name + "_scratch")(sd.seg_len, sd.len)))
             self._finish(4, [d])
         elif op == "PERMUTE":
-            t = TYPE_SUFFIX[ins.typ or "INT"]
+            fn, sfn = ins.x or self.bind(ins, "smp_pe" + TYPE_SUFFIX[ins.typ or "INT"])
             x, idx, sd = st[-3], st[-2], st[-1]
             d = self.new(x.kind, x.len)
-            name = f"smp_pe{t}"
-            self.fn(name)(d.ptr, x.ptr, idx.ptr, sd.ptr, sd.seg_len, sd.len,
-                          self.scratch(self.sfn(name + "_scratch")(sd.seg_len, sd.len)))
+            fn(d.ptr, x.ptr, idx.ptr, sd.ptr, sd.seg_len, sd.len, self.scratch_for(sfn, sd.seg_len, sd.len))
             self._finish(3, [d])
         elif op == "BPERMUTE":
-            t = TYPE_SUFFIX[ins.typ or "INT"]
+            fn, sfn = ins.x or self.bind(ins, "bck_pe" + TYPE_SUFFIX[ins.typ or "INT"])
             x, idx, sds, sdd = st[-4], st[-3], st[-2], st[-1]
             d = self.new(x.kind, idx.len)
-            name = f"bck_pe{t}"
-            self.fn(name)(d.ptr, x.ptr, idx.ptr, sds.ptr, sds.seg_len, sds.len, sdd.ptr, sdd.seg_len, sdd.len,
-                          self.scratch(self.sfn(name + "_scratch")(sds.seg_len, sds.len, sdd.seg_len, sdd.len)))
+            fn(d.ptr, x.ptr, idx.ptr, sds.ptr, sds.seg_len, sds.len, sdd.ptr, sdd.seg_len, sdd.len,
+               self.scratch_for(sfn, sds.seg_len, sds.len, sdd.seg_len, sdd.len))
             self._finish(4, [d])
         elif op == "DPERMUTE":
-            t = TYPE_SUFFIX[ins.typ or "INT"]
+            fn, sfn = ins.x or self.bind(ins, "dpe_pe" + TYPE_SUFFIX[ins.typ or "INT"])
             x, idx, dflt, sds, sdd = st[-5], st[-4], st[-3], st[-2], st[-1]
             if dflt.ref == 1 and not dflt.const:  # the default dies here: permute into it
                 dflt.ref += 1
                 d = dflt
             else:
                 d = self.new(x.kind, dflt.len)
-            name = f"dpe_pe{t}"
-            self.fn(name)(d.ptr, x.ptr, idx.ptr, dflt.ptr, sds.ptr, sds.seg_len, sds.len, sdd.ptr, sdd.seg_len,
-                          sdd.len,
-                          self.scratch(self.sfn(name + "_scratch")(sds.seg_len, sds.len, sdd.seg_len, sdd.len)))
+            fn(d.ptr, x.ptr, idx.ptr, dflt.ptr, sds.ptr, sds.seg_len, sds.len, sdd.ptr, sdd.seg_len, sdd.len,
+               self.scratch_for(sfn, sds.seg_len, sds.len, sdd.seg_len, sdd.len))
             self._finish(5, [d])
         elif op in ("FPERMUTE", "BFPERMUTE"):
             t = TYPE_SUFFIX[ins.typ or "INT"]
@@ -1225,10 +1272,13 @@ class Interpreter:
 
     def _finish(self, nargs, results):
         st = self.stack
-        for v in st[len(st) - nargs:]:
-            self.drop(v)
-        del st[len(st) - nargs:]
-        st.extend(results)
+        k = len(st) - nargs
+        release = self.heap.release
+        for v in st[k:]:
+            v.ref -= 1
+            if v.ref == 0 and not v.const:
+                release(v.ptr, v.cls)
+        st[k:] = results
 
     def _pack(self, ins):
         st = self.stack
@@ -1236,13 +1286,13 @@ class Interpreter:
         x, flg, sd = st[-3], st[-2], st[-1]
         n, m = sd.seg_len, sd.len
         lens = self.new("I", m)
-        self.fn("pk1_lev")(lens.ptr, flg.ptr, sd.ptr, n, m, self.scratch(self.sfn("pk1_lev_scratch")(n, m)))
+        self.fn("pk1_lev")(lens.ptr, flg.ptr, sd.ptr, n, m, self.scratch_for(self.sfn("pk1_lev_scratch"), n, m))
         dsd = self.segdes_from_lengths(lens)
         self.drop(lens)
         d = self.new(x.kind, dsd.seg_len)
         name = f"pk2_le{t}"
         self.fn(name)(d.ptr, x.ptr, flg.ptr, sd.ptr, n, m, dsd.ptr, dsd.seg_len, m,
-                      self.scratch(self.sfn(name + "_scratch")(n, m, dsd.seg_len, m)))
+                      self.scratch_for(self.sfn(name + "_scratch"), n, m, dsd.seg_len, m))
         self._finish(3, [d, dsd])
 
 
