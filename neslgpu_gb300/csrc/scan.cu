@@ -361,14 +361,14 @@ template <int ITEMS> struct Engine<AddD, ITEMS> {
   }
 };
 
-// Float64 + reductions of short segments (the CHAIN form of the kernel,
-// chosen when segments average under RED_CHAIN_MEAN elements): a warp in
-// which some thread ends at least two segments sums its pieces with one FP64
-// add per item instead of a fixed-point pass per segment end.  At 2^28,
-// geometric(4) segments 2.98 -> 1.14 ms, geometric(64) 1.12 -> 1.01 ms; the
-// log-normal(5,2) bench segments (about 1100 elements on average) keep the
-// plain form, which the chain's code alone slows by 2-4 %.
-constexpr long RED_CHAIN_MEAN = 256;
+// Float64 + reductions of segments averaging under RED_CHAIN_MEAN elements
+// (the CHAIN form of the kernel) take the one pass of the other operators,
+// one FP64 add per item, instead of a fixed-point fold and another
+// fixed-point pass per segment end (chained in warps with many ends before).
+// add_red at 2^25, that / one pass, us: mean 2 178 / 147, 8 170 / 137, 64 155 /
+// 126, 128 149 / 121, 255 138 / 119; folding alone at 257 123, at 1100 99, where
+// one pass takes 118 and 113, so the line lies between.
+constexpr long RED_CHAIN_MEAN = 350;
 // Reductions: a thread's float64 + fold split between the integer pipes
 // (the first GCVL_RED_FX_ITEMS items, fixed point) and the FP64 pipe (the
 // rest, an add chain), so that neither carries the whole fold; 14 of 16
@@ -616,12 +616,12 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
 
   int tf;
   T tv;
-  // Reductions other than float64 + take one pass over the thread's items:
-  // the results of segments that start and end among them are final at
-  // once; the first segment end, whose segment began before these items,
-  // waits for the earlier threads' prefix (first_s, first_v).  Float64 +
+  // Reductions take one pass over the thread's items: the results of segments
+  // that start and end among them are final at once; the first segment end,
+  // whose segment began before these items, waits for the earlier threads'
+  // prefix (first_s, first_v).  Float64 + over longer segments (not CHAIN)
   // folds in fixed point per piece below.
-  constexpr bool ONE_PASS = SEG && MODE == M_REDUCE && !std::is_same<Op, AddD>::value;
+  constexpr bool ONE_PASS = SEG && MODE == M_REDUCE && (!std::is_same<Op, AddD>::value || CHAIN);
   int first_s = -1;
   T first_v = Op::ident();
   if constexpr (ONE_PASS) {
@@ -735,82 +735,31 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
       put(first_s, Op::apply(run, first_v));
       if (!pf) a.lead[tile] = first_s;  // began in an earlier tile
     }
-  } else {  // M_REDUCE: results at segment ends
-    // float64 +: pieces between heads, each summed in fixed point.  Element
-    // i ends a non-empty segment exactly when element i+1 is a head (or past
-    // the end): only those positions are visited (mostly none).  Whether the
-    // warp chains its items is decided by every lane, those past the
-    // vector's end too (they hold no ends): a warp vote must not name lanes
-    // that are elsewhere.
-    unsigned ends = 0;
-    bool chain_warp = false;
-    if constexpr (std::is_same<Op, AddD>::value) {
-      if (cnt > 0) {
-        const int kn = k0 + cnt;
-        const unsigned nh = kn >= a.n ? 1u : (__ldg(a.sv.bits + (kn >> 5)) >> (kn & 31)) & 1u;
-        ends = ((heads >> 1) | (nh << (cnt - 1))) & (cnt >= 32 ? ~0u : ((1u << cnt) - 1u));
-      }
-      if (CHAIN) chain_warp = __any_sync(0xffffffffu, __popc(ends) >= 2);
-    }
+  } else if constexpr (MODE == M_REDUCE && SEG) {  // float64 + over longer segments: results at segment ends
+    // pieces between heads, each summed in fixed point.  Element i ends a
+    // non-empty segment exactly when element i+1 is a head (or past the end):
+    // only those positions are visited (mostly none).
     if (cnt > 0) {
+      const int kn = k0 + cnt;
+      const unsigned nh = kn >= a.n ? 1u : (__ldg(a.sv.bits + (kn >> 5)) >> (kn & 31)) & 1u;
+      unsigned ends = ((heads >> 1) | (nh << (cnt - 1))) & (cnt >= 32 ? ~0u : ((1u << cnt) - 1u));
       const int m = a.sv.m;
       if (k0 == 0)
         for (int s = 0; s < s0; s++) put(s, Op::init());
       int s = s0;
       int end = off(s + 1);
-      if constexpr (std::is_same<Op, AddD>::value) {
-        if (chain_warp) {
-          // short segments: one FP64 add per item beats a fixed-point pass
-          // per segment end (each a separate sum of up to 16 items)
-          double r = run;
-#pragma unroll
-          for (int i = 0; i < ITEMS; i++) {
-            if (i < cnt) {
-              if ((heads >> i) & 1u) r = 0.0;
-              r = __dadd_rn(r, x[i]);
-              if ((ends >> i) & 1u) {
-                put(s, r);
-                if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
-                int s2 = s + 1;
-                while (s2 < m && off(s2 + 1) == end) { put(s2, 0.0); ++s2; }
-                s = s2;
-                if (s < m) end = off(s + 1);
-              }
-            }
-          }
-          ends = 0;
-        }
-        int ps = 0;
-        while (ends) {
-          const int i = __ffs(ends) - 1;
-          ends &= ends - 1;
-          {
-            double pv2 = fx_range<ITEMS>(x, ps, i + 1);
-            put(s, ((heads >> ps) & 1u) ? pv2 : AddD::apply(run, pv2));
-            if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
-            int s2 = s + 1;
-            while (s2 < m && off(s2 + 1) == end) { put(s2, 0.0); ++s2; }
-            s = s2;
-            if (s < m) end = off(s + 1);
-            ps = i + 1;
-          }
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < ITEMS; i++) {
-          if (i < cnt) {
-            if ((heads >> i) & 1u) run = Op::init();
-            run = Op::apply(run, x[i]);
-            if (k0 + i + 1 == end) {
-              put(s, run);
-              if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
-              int s2 = s + 1;
-              while (s2 < m && off(s2 + 1) == end) { put(s2, Op::init()); ++s2; }
-              s = s2;
-              if (s < m) end = off(s + 1);
-            }
-          }
-        }
+      int ps = 0;
+      while (ends) {
+        const int i = __ffs(ends) - 1;
+        ends &= ends - 1;
+        const double pv2 = fx_range<ITEMS>(x, ps, i + 1);
+        put(s, ((heads >> ps) & 1u) ? pv2 : AddD::apply(run, pv2));
+        if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
+        int s2 = s + 1;
+        while (s2 < m && off(s2 + 1) == end) { put(s2, 0.0); ++s2; }
+        s = s2;
+        if (s < m) end = off(s + 1);
+        ps = i + 1;
       }
     }
   }

@@ -292,3 +292,15 @@ def test_float_sums_either_side_of_the_ring(gpu, oracle, name, n):
     else:
         g, o = ops.scan_u(gpu, name, x), ops.scan_u(oracle, name, x)
     assert np.all(np.abs(g - o) <= 1e-12 * np.maximum(mag, np.abs(o)))
+
+
+@pytest.mark.parametrize("mean", [1, 2, 15, 16, 17, 349, 350, 351])
+def test_float_sums_of_even_segments(gpu, oracle, mean):
+    """Either side of the mean from which the sums fold in fixed point; rows hold 16 elements, tiles 2048."""
+    r = W.rng(mean)
+    m = 700_003 // mean
+    lens = np.full(m, mean, dtype=np.int32)
+    x = W.float64_normal(r, m * mean) * 2.0 ** r.integers(-40, 40, size=m * mean)
+    mag = np.add.reduceat(np.abs(x), np.arange(m) * mean)
+    g, o = ops.reduce_e(gpu, "add_red", x, lens), ops.reduce_e(oracle, "add_red", x, lens)
+    assert np.all(np.abs(g - o) <= 1e-12 * mag)
