@@ -363,44 +363,15 @@ template <int ITEMS> struct Engine<AddD, ITEMS> {
 
 // Float64 + reductions of segments averaging under RED_CHAIN_MEAN elements
 // (the CHAIN form of the kernel) take the one pass of the other operators,
-// one FP64 add per item, instead of a fixed-point fold and another
-// fixed-point pass per segment end (chained in warps with many ends before).
-// add_red at 2^25, that / one pass, us: mean 2 178 / 147, 8 170 / 137, 64 155 /
-// 126, 128 149 / 121, 255 138 / 119; folding alone at 257 123, at 1100 99, where
-// one pass takes 118 and 113, so the line lies between.
-constexpr long RED_CHAIN_MEAN = 350;
-// Reductions: a thread's float64 + fold split between the integer pipes
-// (the first GCVL_RED_FX_ITEMS items, fixed point) and the FP64 pipe (the
-// rest, an add chain), so that neither carries the whole fold; 14 of 16
-// measured best (8 of 16: 16 % slower, 16 of 16: 3 %).  The segmented
-// reduction has no per-element output work to keep the FP64 pipe busy.
-#ifndef GCVL_RED_FX_ITEMS
-#define GCVL_RED_FX_ITEMS 14
+// one FP64 add per item, in every warp; longer ones fold in fixed point the
+// warps in which no segment starts or ends.  A fold in every warp, with
+// another fixed-point sum per segment end, took at 2^25, and now, us: mean 2
+// 178 / 147, 8 170 / 137, 64 155 / 126, 257 123 / 115, 1100 99 / 90, 10^6 70 /
+// 69.  The line: mean 64 126 in one pass against 128, 300 118 against 115.
+#ifndef GCVL_RED_CHAIN_MEAN
+#define GCVL_RED_CHAIN_MEAN 128
 #endif
-template <int ITEMS>
-__device__ __forceinline__ void agg_add_split(const double (&x)[ITEMS], unsigned heads, int cnt, int &tf,
-                                              double &tv) {
-  constexpr int H = GCVL_RED_FX_ITEMS < ITEMS ? GCVL_RED_FX_ITEMS : ITEMS;  // items in fixed point
-  tf = heads != 0;
-  tv = AddD::ident();
-  if (__all_sync(0xffffffffu, heads == 0 && cnt == ITEMS)) {
-    // the whole warp folds full rows without segment starts: no per-item tests
-    const double lo = fx_range_part<ITEMS, 0, H>(x, 0, ITEMS);
-    double hi = -0.0;
-#pragma unroll
-    for (int i = H; i < ITEMS; i++) hi = __dadd_rn(hi, x[i]);
-    tv = __dadd_rn(lo, hi);
-    return;
-  }
-  if (cnt <= 0) return;
-  const int from = heads ? 31 - __clz((int)heads) : 0;
-  const double lo = fx_range_part<ITEMS, 0, H>(x, from, cnt);
-  double hi = -0.0;
-#pragma unroll
-  for (int i = H; i < ITEMS; i++)
-    if (i >= from && i < cnt) hi = __dadd_rn(hi, x[i]);
-  tv = __dadd_rn(lo, hi);
-}
+constexpr long RED_CHAIN_MEAN = GCVL_RED_CHAIN_MEAN;
 
 // The CTA has TT compute threads (one 128-byte row each) plus one look-back
 // warp.  The look-back warp issues the tile's TMA load and at once starts
@@ -619,12 +590,24 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
   // Reductions take one pass over the thread's items: the results of segments
   // that start and end among them are final at once; the first segment end,
   // whose segment began before these items, waits for the earlier threads'
-  // prefix (first_s, first_v).  Float64 + over longer segments (not CHAIN)
-  // folds in fixed point per piece below.
-  constexpr bool ONE_PASS = SEG && MODE == M_REDUCE && (!std::is_same<Op, AddD>::value || CHAIN);
+  // prefix (first_s, first_v).  Float64 + over longer segments (FOLD) does so
+  // only in warps where a segment starts or ends; the others (their rows are
+  // full, or all past the end) fold theirs in fixed point, all 16 items (the
+  // last two in FP64 as well: 95 us against 90 at 1100 elements a segment).
+  constexpr bool FOLD = MODE == M_REDUCE && std::is_same<Op, AddD>::value && !CHAIN;
   int first_s = -1;
   T first_v = Op::ident();
-  if constexpr (ONE_PASS) {
+  bool folded = false;
+  if constexpr (FOLD) {
+    const int kn = k0 + cnt;
+    const bool nh = cnt > 0 && (kn >= a.n || ((__ldg(a.sv.bits + (kn >> 5)) >> (kn & 31)) & 1u));
+    folded = !__any_sync(0xffffffffu, heads != 0 || nh);
+    if (folded) {
+      tf = 0;
+      tv = cnt > 0 ? fx_range<ITEMS>(x, 0, ITEMS) : AddD::ident();
+    }
+  }
+  if (SEG && MODE == M_REDUCE && !folded) {
     T r = Op::ident();
     bool started = false;
     if (cnt > 0) {
@@ -651,24 +634,26 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
     }
     tf = heads != 0;
     tv = r;
-  } else if constexpr (MODE == M_REDUCE && std::is_same<Op, AddD>::value) {
-    agg_add_split<ITEMS>(x, heads, cnt, tf, tv);
-  } else {
-    Engine<Op, ITEMS>::agg(x, heads, cnt, tf, tv);
   }
+  if (MODE == M_SCAN) Engine<Op, ITEMS>::agg(x, heads, cnt, tf, tv);
 
-  // warp inclusive scan of (head, value)
-  int f = tf;
-  T v = tv;
+  // warp inclusive scan of (head, value); a folded warp only needs its total
+  int f = tf, ef = 0;
+  T v = tv, ev = Op::ident();
+  if (folded) {
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    int f2 = shfl_up(f, d);
-    T v2 = shfl_up(v, d);
-    if (lane >= d) { v = f ? v : Op::apply(v2, v); f |= f2; }
+    for (int d = 1; d < 32; d <<= 1) v = Op::apply(shfl_up(v, d), v);  // lane 31's holds every lane
+  } else {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      int f2 = shfl_up(f, d);
+      T v2 = shfl_up(v, d);
+      if (lane >= d) { v = f ? v : Op::apply(v2, v); f |= f2; }
+    }
+    ef = shfl_up(f, 1);
+    ev = shfl_up(v, 1);
+    if (lane == 0) { ef = 0; ev = Op::ident(); }
   }
-  int ef = shfl_up(f, 1);
-  T ev = shfl_up(v, 1);
-  if (lane == 0) { ef = 0; ev = Op::ident(); }
   if (lane == 31) { s_wf[warp] = f; s_wv[warp] = v; }
   named_sync(2, TT);
 
@@ -730,38 +715,9 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
       bulk_commit();
       bulk_wait_read_all();
     }
-  } else if constexpr (ONE_PASS) {  // the one result still lacking the earlier part
-    if (first_s >= 0) {
-      put(first_s, Op::apply(run, first_v));
-      if (!pf) a.lead[tile] = first_s;  // began in an earlier tile
-    }
-  } else if constexpr (MODE == M_REDUCE && SEG) {  // float64 + over longer segments: results at segment ends
-    // pieces between heads, each summed in fixed point.  Element i ends a
-    // non-empty segment exactly when element i+1 is a head (or past the end):
-    // only those positions are visited (mostly none).
-    if (cnt > 0) {
-      const int kn = k0 + cnt;
-      const unsigned nh = kn >= a.n ? 1u : (__ldg(a.sv.bits + (kn >> 5)) >> (kn & 31)) & 1u;
-      unsigned ends = ((heads >> 1) | (nh << (cnt - 1))) & (cnt >= 32 ? ~0u : ((1u << cnt) - 1u));
-      const int m = a.sv.m;
-      if (k0 == 0)
-        for (int s = 0; s < s0; s++) put(s, Op::init());
-      int s = s0;
-      int end = off(s + 1);
-      int ps = 0;
-      while (ends) {
-        const int i = __ffs(ends) - 1;
-        ends &= ends - 1;
-        const double pv2 = fx_range<ITEMS>(x, ps, i + 1);
-        put(s, ((heads >> ps) & 1u) ? pv2 : AddD::apply(run, pv2));
-        if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
-        int s2 = s + 1;
-        while (s2 < m && off(s2 + 1) == end) { put(s2, 0.0); ++s2; }
-        s = s2;
-        if (s < m) end = off(s + 1);
-        ps = i + 1;
-      }
-    }
+  } else if (first_s >= 0) {  // the one result still lacking the earlier part
+    put(first_s, Op::apply(run, first_v));
+    if (!pf) a.lead[tile] = first_s;  // began in an earlier tile
   }
   if constexpr (STAGE) {
     if (staged) {
