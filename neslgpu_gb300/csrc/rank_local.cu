@@ -8,11 +8,11 @@
 // (a non-decreasing map, so buckets are in key order); the elements are
 // placed bucket by bucket in shared memory, and an element's rank is its
 // bucket's start plus the keys before its own inside the bucket, ties by
-// index (the stable order of nesl/cvl/serial/rank.c:49-362).  With keys spread over their range a bucket holds one or two
-// elements whatever the segment's length.  A CTA whose buckets came out
-// crowded (few distinct keys, clustered keys) sorts its keys instead with
-// stable 8-bit digit passes in shared memory, skipping the digits on which
-// all its keys agree.
+// index (the stable order of nesl/cvl/serial/rank.c:49-362).  With keys
+// spread over their range a bucket holds one or two elements whatever the
+// segment's length.  A CTA whose buckets came out crowded (few distinct keys,
+// clustered keys) sorts its keys instead with stable 8-bit digit passes in
+// shared memory, skipping the digits on which all its keys agree.
 //
 // Segments longer than LR_MAX are numbered and given room in a compacted
 // vector, which the digit passes of rank.cu then sort.
@@ -24,11 +24,11 @@ namespace gcvl {
 constexpr int LR_WARPS = LR_BLOCK / 32;
 constexpr int LR_STEPS = LR_CAP / LR_BLOCK;  // elements of a thread in a full CTA
 constexpr int LR_WORDS = LR_CAP / 32 + 1;    // head-bit words: a full CTA's, and the one that may end it
-#ifndef GCVL_LR_MINB
-#define GCVL_LR_MINB 3
-#endif
 constexpr size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
-template <class K> constexpr int lr_minb() { return sizeof(K) == 4 ? GCVL_LR_MINB : 2; }
+// CTAs an SM is asked to hold: all its threads with 4-byte keys (rku_sez at
+// 2^24 with segments of 64 by 2 CTAs 227.6 us, by 3 207.2, by 4 203.1); two
+// with 8-byte keys, whose tile takes twice the shared memory.
+template <class K> constexpr int lr_minb() { return sizeof(K) == 4 ? 4 : 2; }
 // Buckets are compared element by element while that costs less than the
 // digit passes: about 10 instructions per comparison against 45 per element
 // and digit.
@@ -107,9 +107,9 @@ template <class K> constexpr size_t lr_smem() {
 }
 
 // Bound by issue: about 300 instructions per element and lane (79 % of issue
-// slots), 2^24 int keys in geometric(64) segments 164 us where the bytes take
-// 20; the whole call 1284 -> 207 us against sorting by (segment, key)
-// globally (7 digit passes).  The shape: 512 threads and three CTAs per SM;
+// slots), 2^24 int keys in geometric(64) segments 160 us where the bytes take
+// 20; the whole call 1284 -> 203 us against sorting by (segment, key)
+// globally (7 digit passes).  The shape: 512 threads and four CTAs per SM;
 // with 256 threads each holding rows of eight consecutive keys in shared
 // memory 280 us, with bucket ends found in a bit map of bucket starts instead
 // of from the places 219 us.
