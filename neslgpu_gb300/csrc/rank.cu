@@ -553,6 +553,96 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
   }
 }
 
+// Waits until all CTAs of a resident grid have arrived as often as this one:
+// what any of them stored before, all may load afterwards.  Returns the
+// CTA's number, read from memory after the wait, so that loads whose address
+// comes from it cannot be moved ahead; negative when the bounded wait, or any
+// wait before it, gave up (the next pass would follow indices nobody wrote).
+__device__ __forceinline__ int rk_meet(unsigned *count, unsigned arrivals, unsigned *status, int limit) {
+  __shared__ volatile int s_cta;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1, it = 0;
+    __threadfence();
+    atomicAdd(count, 1u);
+    while (*(volatile unsigned *)count < arrivals) {
+      if (++it >= limit) { ok = 0; atomicOr(status, DEV_TIMEOUT); break; }
+      if (it > 64) __nanosleep(32);
+    }
+    __threadfence();
+    s_cta = ok && !(*(volatile unsigned *)status & DEV_TIMEOUT) ? (int)blockIdx.x : -1;
+  }
+  __syncthreads();
+  return s_cta;
+}
+
+// The digit passes over the long segments, whose number and elements only
+// the device knows: by the key, then by the segment number.
+template <class K> struct LongArgs {
+  K *key[2];                // pass q reads [q & 1] and writes the other
+  unsigned *idx[2], *aux[2];
+  int *rank; const int *segbase;
+  const unsigned *hist;
+  unsigned *state[3], *meet;
+  const unsigned long long *total;
+  int seg_passes;
+  unsigned *status;
+  int spin_limit;
+};
+// One cooperative launch that meets between passes.  There are usually no
+// long segments, and then a launch for every pass was most of a call: in
+// segments of 64, a launch a pass / this, us: 2^16 int keys 37 / 22, 2^20
+// float64 71 / 34; with long segments, 2^19 int bimodal 80 / 71, 2^20 float64
+// log-normal 161 / 144.  In the larger tiles of longer vectors the passes
+// themselves ran 2-5 % slower here (2^23 float64 log-normal 652 / 683, with
+// tickets) and stay apart.
+// All CTAs are resident and take their tiles in increasing order, so a tile's
+// look-back waits only for tiles that are being ranked: no tickets, whose two
+// round trips a pass the meeting would not make up for.  None of a pass's
+// loads of an earlier one's output is a read-only load.
+template <class K, int ITEMS>
+__global__ void __launch_bounds__(RK_BLOCK, GCVL_RK_MINB) k_rank_long(const __grid_constant__ LongArgs<K> l) {
+  const int n = (int)(unsigned)*(volatile const unsigned long long *)l.total;
+  if (n == 0) return;  // every CTA alike
+  const int tiles = (int)(((long)n + RK_BLOCK * ITEMS - 1) / (RK_BLOCK * ITEMS));
+  const int ctas = min(tiles, (int)gridDim.x);
+  if ((int)blockIdx.x >= ctas) return;
+  constexpr int P = sizeof(K);
+  const int passes = P + l.seg_passes;
+  auto common = [&](auto &a, int q) {
+    a.vin = l.idx[q & 1]; a.vout = l.idx[~q & 1];
+    a.hist = l.hist + q * 256;
+    a.state = l.state[q % 3];
+    a.clear = q > 0 && q < passes - 1 ? l.state[(q + 2) % 3] : nullptr;
+    a.status = l.status; a.spin_limit = l.spin_limit;
+  };
+  int first = blockIdx.x;
+#pragma unroll 1
+  for (int q = 0; q < passes; q++) {
+    if (q > 0 && (first = rk_meet(l.meet, (unsigned)(q * ctas), l.status, l.spin_limit)) < 0) return;
+#pragma unroll 1
+    for (int tile = first; tile < tiles; tile += ctas) {
+      if (q < P) {
+        PassArgs<K, unsigned> a{};
+        common(a, q);
+        a.kin = l.key[q & 1]; a.kout = l.key[~q & 1];
+        a.ain = l.aux[q & 1]; a.aout = l.aux[~q & 1];
+        a.shift = 8 * q;
+        radix_tile<K, unsigned, true, IN_ARRAYS, OUT_ARRAYS, ITEMS>(a, n, tile);
+      } else {  // the segment number is the key, indices ride along
+        PassArgs<unsigned, unsigned> a{};
+        common(a, q);
+        a.kin = q == P ? l.aux[0] : (const unsigned *)l.key[q & 1];
+        a.kout = (unsigned *)l.key[~q & 1];
+        a.rank = l.rank; a.segbase = l.segbase; a.shift = 8 * (q - P);
+        if (q < passes - 1) radix_tile<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS, ITEMS>(a, n, tile);
+        else radix_tile<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, ITEMS>(a, n, tile);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // d[key[i]] = val[i], streaming over pairs that a partition pass grouped by
 // output window
 template <class V>
@@ -818,10 +908,30 @@ inline int rk_tile(long n) {
 }
 template <class K, class V, bool AUX, int IN, int OUT, bool DYN> void launch_pass(const PassArgs<K, V> &a) {
   if (a.n > RK_SMALL_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_LARGE, DYN>(a);
-  else if constexpr (OUT != OUT_WIN) {
+  else if constexpr (OUT != OUT_WIN && !DYN) {
     if (a.n > RK_TINY_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_SMALL, DYN>(a);
     else launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_TINY, DYN>(a);
   }
+}
+template <class K, int ITEMS> void launch_long_items(LongArgs<K> l, int n) {
+  constexpr size_t sm =
+      std::max(pass_smem<K, unsigned, true, ITEMS>(), pass_smem<unsigned, unsigned, false, ITEMS>());
+  static int per_sm = 0;  // of a cooperative launch, whose CTAs are all resident
+  if (per_sm < 1) {
+    GCVL_CK(cudaFuncSetAttribute(k_rank_long<K, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    int nb = 0;
+    if (!GCVL_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_rank_long<K, ITEMS>, RK_BLOCK, sm))) return;
+    per_sm = std::max(nb, 1);
+  }
+  const int grid = std::min(ceil_div(n, RK_BLOCK * ITEMS), per_sm * st().sm_count);
+  void *args[] = {&l};
+  GCVL_CK(cudaLaunchCooperativeKernel((const void *)k_rank_long<K, ITEMS>, dim3(grid), dim3(RK_BLOCK), args, sm,
+                                      stream()));
+  launch_check("k_rank_long");
+}
+template <class K> void launch_long(const LongArgs<K> &l, int n) {
+  if (n > RK_TINY_MAX) launch_long_items<K, RK_ITEMS_SMALL>(l, n);
+  else launch_long_items<K, RK_ITEMS_TINY>(l, n);
 }
 static_assert(RK_SMALL_MAX <= RK_DIRECT_MAX, "windows only for large tiles");
 
@@ -1047,7 +1157,7 @@ inline RankLayout rank_layout(int n, int is_double, int seg) {
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += align_up(bytes, 256); return at; };
   L.hist = take(RK_MAXPASS * 256 * 4);  // these three are cleared together
-  L.counter = take(RK_MAXPASS * 4);
+  L.counter = take((RK_MAXPASS + 1) * 4);  // tickets, and the long segments' meetings
   L.lsum = take(8);
   L.state = take(rk_state_bytes(n) * 3);
   L.key_a = take((size_t)n * ks);
@@ -1094,9 +1204,10 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
   unsigned *iA = (unsigned *)(mem + L.idx_a), *iB = (unsigned *)(mem + L.idx_b);
   unsigned *aA = (unsigned *)(mem + L.aux_a), *aB = (unsigned *)(mem + L.aux_b);
   const int key_passes = (int)sizeof(K);
-  int seg_passes = 0;
+  const bool direct = n <= RK_DIRECT_MAX;
+  const int wshift = window_shift(n);
+  unsigned *pidx = nullptr, *ppos = nullptr, *wstate = nullptr;
   const unsigned long long *total = nullptr;
-  const int *segbase = nullptr;
   if (seg) {
     LongSegs ls;
     ls.total = (unsigned long long *)(mem + L.lsum);
@@ -1107,12 +1218,58 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
     if (n <= LR_MAX) return;  // no segment can be longer
     // the long segments, if there are any: the kernels below return at once otherwise
     total = ls.total;
-    segbase = ls.base;
-    seg_passes = std::max(1, (bit_length((unsigned)(n / (LR_MAX + 1) - 1)) + 7) / 8);
+    const int seg_passes = std::max(1, (bit_length((unsigned)(n / (LR_MAX + 1) - 1)) + 7) / 8);
     const int pg = std::min(S.sm_count * 8, lr_tiles(n));
     k_rank_prep_long<K><<<pg, RK_BLOCK, 0, S.stream>>>((const K *)s, n, up, sv, ls, seg_passes, (K *)kA, iA, aA, hist,
                                                        state[0], (long)(state_bytes / 4), rk_tile(n));
     launch_check("k_rank_prep_long");
+    LongArgs<K> l{};
+    l.key[0] = (K *)kA; l.key[1] = (K *)kB;
+    l.idx[0] = iA; l.idx[1] = iB;
+    l.aux[0] = aA; l.aux[1] = aB;
+    l.rank = (int *)d; l.segbase = ls.base; l.hist = hist;
+    for (int b = 0; b < 3; b++) l.state[b] = state[b];
+    l.meet = counters + RK_MAXPASS;
+    l.total = total; l.seg_passes = seg_passes;
+    l.status = S.d_status; l.spin_limit = S.spin_limit;
+    if (n <= RK_SMALL_MAX) {
+      launch_long<K>(l, n);
+      return;
+    }
+    const int passes = key_passes + seg_passes;
+    for (int q = 0; q < passes; q++) {
+      const bool final = (q == passes - 1);
+      auto common = [&](auto &a) {
+        a.vin = l.idx[q & 1]; a.vout = l.idx[~q & 1];
+        a.hist = hist + q * 256; a.counter = counters + q;
+        a.state = state[q % 3]; a.clear = q > 0 && !final ? state[(q + 2) % 3] : nullptr;
+        a.total = total; a.n = n; a.status = S.d_status; a.spin_limit = S.spin_limit;
+      };
+      if (q < key_passes) {
+        PassArgs<K, unsigned> a{};
+        common(a);
+        a.kin = l.key[q & 1]; a.kout = l.key[~q & 1];
+        a.ain = l.aux[q & 1]; a.aout = l.aux[~q & 1];
+        a.shift = 8 * q;
+        launch_pass<K, unsigned, true, IN_ARRAYS, OUT_ARRAYS, true>(a);
+      } else {
+        // segment passes: the segment number is the key, indices ride along
+        PassArgs<unsigned, unsigned> a{};
+        common(a);
+        a.kin = q == key_passes ? aA : (const unsigned *)l.key[q & 1];
+        a.kout = (unsigned *)l.key[~q & 1];
+        a.segbase = ls.base; a.shift = 8 * (q - key_passes);
+        if (final) {  // the pairs by window take the buffers the last pass does not read
+          a.rank = (int *)d;
+          a.pidx = pidx = a.vout;
+          a.ppos = ppos = a.kout;
+          a.wstate = wstate = state[(q + 1) % 3]; a.wshift = wshift;
+        }
+        if (!final) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS, true>(a);
+        else if (direct) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, true>(a);
+        else launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_WIN, true>(a);
+      }
+    }
   } else {
     // at least 16 keys a thread: every CTA adds its histograms to the vector's
     // with an atomic per bin (2^20 keys by 1216 CTAs 14.6 us, by 256 5)
@@ -1120,55 +1277,30 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
     k_rank_prep<K><<<pg, RK_BLOCK, 0, S.stream>>>((const K *)s, n, up, hist, (uint4 *)state[0],
                                                   (long)(3 * state_bytes / 16));
     launch_check("k_rank_prep");
-  }
-
-  const int passes = key_passes + seg_passes;
-  const bool direct = n <= RK_DIRECT_MAX;
-  const int wshift = window_shift(n);
-  unsigned *pidx = nullptr, *ppos = nullptr, *wstate = nullptr;
-  for (int q = 0; q < passes; q++) {
-    const bool final = (q == passes - 1);
-    if (final) {  // the pairs by window take the buffers the last pass does not read
-      pidx = iB;
-      ppos = (unsigned *)kB;
-      wstate = state[(q + 1) % 3];
-    }
-    auto common = [&](auto &a) {
-      a.vin = iA;
-      a.vout = iB;
-      a.rank = (int *)d; a.pidx = pidx; a.ppos = ppos;
+    for (int q = 0; q < key_passes; q++) {
+      const bool final = (q == key_passes - 1);
+      PassArgs<K, unsigned> a{};
+      a.kin = (const K *)kA; a.kout = (K *)kB;
+      a.vin = iA; a.vout = iB;
+      a.src = s; a.up = up; a.shift = 8 * q;
       a.hist = hist + q * 256; a.counter = counters + q;
       a.state = state[q % 3]; a.clear = q > 0 && !final ? state[(q + 2) % 3] : nullptr;
-      a.wstate = wstate; a.wshift = wshift;
-      a.total = total; a.n = n; a.status = S.d_status; a.spin_limit = S.spin_limit;
-    };
-    if (q < key_passes) {
-      PassArgs<K, unsigned> a{};
-      common(a);
-      a.kin = (const K *)kA; a.kout = (K *)kB; a.ain = aA; a.aout = aB;
-      a.src = s; a.up = up; a.shift = 8 * q;
-      if (seg) launch_pass<K, unsigned, true, IN_ARRAYS, OUT_ARRAYS, true>(a);
-      else if (q == 0) launch_pass<K, unsigned, false, IN_SRC, OUT_ARRAYS, false>(a);
+      a.n = n; a.status = S.d_status; a.spin_limit = S.spin_limit;
+      if (final) {  // the pairs by window take the buffers the last pass does not read
+        a.rank = (int *)d;
+        a.pidx = pidx = iB;
+        a.ppos = ppos = (unsigned *)kB;
+        a.wstate = state[(q + 1) % 3]; a.wshift = wshift;
+      }
+      if (q == 0) launch_pass<K, unsigned, false, IN_SRC, OUT_ARRAYS, false>(a);
       else if (!final) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_ARRAYS, false>(a);
       else if (direct) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_RANK, false>(a);
       else launch_pass<K, unsigned, false, IN_ARRAYS, OUT_WIN, false>(a);
-    } else {
-      // segment passes: the segment number is the key, indices ride along
-      PassArgs<unsigned, unsigned> a{};
-      common(a);
-      a.kin = q == key_passes ? aA : (const unsigned *)kA;
-      a.kout = (unsigned *)kB;
-      a.segbase = segbase; a.shift = 8 * (q - key_passes);
-      if (!final) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS, true>(a);
-      else if (direct) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, true>(a);
-      else launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_WIN, true>(a);
-    }
-    if (!final) {
       std::swap(kA, kB);
       std::swap(iA, iB);
-      if (q < key_passes) std::swap(aA, aB);
     }
   }
+
   if (!direct) {
     if (seg)
       k_rank_scatter<true><<<sc_grid(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, total, wstate,

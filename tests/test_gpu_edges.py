@@ -91,6 +91,32 @@ def test_rank_long_segments_by_window(gpu, oracle, name, n):
     assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
 
 
+@pytest.mark.parametrize("n", [4097, 1 << 18, (1 << 18) + 1, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("name", ["rkd_lez", "rku_led"])
+def test_rank_long_segments_captured(gpu, oracle, name, n):
+    """The passes over the long segments inside a CUDA graph, replayed on other keys, in each of their tile sizes
+    (up to 2^20 elements in one launch that meets between passes); then the same call outside it."""
+    r = W.rng(n + 3)
+    lens = np.array([2049, 0, 7, n - 2056], dtype=np.int32)
+    if n == 4097:
+        lens = np.array([2048, 2049], dtype=np.int32)
+    c, t = gpu.cvl, name[-1]
+    x = [_keys(r, n, t, "uniform"), _keys(r, n, t, "few")]
+    sd, _, m = gpu.segd(lens)
+    k, d = gpu.vec(x[0], t), gpu.out(n, "z")
+    scr = gpu.units(gpu.fn(name + "_scratch")(n, m))
+    assert c.gcvl_graph_begin() == 0
+    gpu.fn(name)(d.ptr, k.ptr, sd.ptr, n, m, scr.ptr)
+    g = c.gcvl_graph_end()
+    for keys in x:
+        k.upload(keys)
+        c.gcvl_graph_launch(g)
+        assert np.array_equal(gpu.get(d, n), ops.rank_e(oracle, name, keys, lens))
+    c.gcvl_graph_destroy(g)
+    assert np.array_equal(ops.rank_e(gpu, name, x[0], lens), ops.rank_e(oracle, name, x[0], lens))
+    assert c.gcvl_sync() == 0
+
+
 # ------------------------------------------------------------------ puts ---
 # the owner passes take 2048 elements a CTA, up to 3 * 2^24 destinations
 def _put_case(r, n_s, n_d, order):
