@@ -222,7 +222,6 @@ template <class K, class V> struct PassArgs {
   unsigned *wstate;                   // OUT_WIN: [tiles][256] look-back words of the window counts
   int wshift;                         // OUT_WIN: window of v = v >> wshift
   unsigned *counter;
-  const unsigned long long *total;    // DYN: the vector's length is the low word
   int n, shift;
   unsigned *status;
   int spin_limit;
@@ -527,30 +526,13 @@ __device__ __forceinline__ void radix_tile(const PassArgs<K, V> &a, const int n,
   }
 }
 
-// One tile per CTA, taken in ticket order.  DYN: the vector's length is only
-// known on the device (long segments, usually none), so a resident grid
-// takes tiles until there are no more and costs one empty launch otherwise
-// (a grid for the longest possible vector: 5-7 us of CTAs that return).
-template <class K, class V, bool AUX, int IN, int OUT, int ITEMS, bool DYN>
+// One tile per CTA, taken in ticket order.
+template <class K, class V, bool AUX, int IN, int OUT, int ITEMS>
 __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(PassArgs<K, V> a) {
   __shared__ unsigned s_tile;
-  if constexpr (DYN) {
-    const long n = (long)(unsigned)*(volatile const unsigned long long *)a.total;
-    const int tiles = (int)((n + RK_BLOCK * ITEMS - 1) / (RK_BLOCK * ITEMS));
-    if ((int)blockIdx.x >= tiles) return;
-    while (true) {
-      if (threadIdx.x == 0) s_tile = atomicAdd(a.counter, 1u);
-      __syncthreads();
-      const int tile = (int)s_tile;
-      if (tile >= tiles) return;
-      radix_tile<K, V, AUX, IN, OUT, ITEMS>(a, (int)n, tile);
-      __syncthreads();
-    }
-  } else {
-    if (threadIdx.x == 0) s_tile = atomicAdd(a.counter, 1u);
-    __syncthreads();
-    radix_tile<K, V, AUX, IN, OUT, ITEMS>(a, a.n, (int)s_tile);
-  }
+  if (threadIdx.x == 0) s_tile = atomicAdd(a.counter, 1u);
+  __syncthreads();
+  radix_tile<K, V, AUX, IN, OUT, ITEMS>(a, a.n, (int)s_tile);
 }
 
 // Waits until all CTAs of a resident grid have arrived as often as this one:
@@ -585,17 +567,15 @@ template <class K> struct LongArgs {
   const unsigned *hist;
   unsigned *state[3], *meet;
   const unsigned long long *total;
-  int seg_passes;
+  int seg_passes, direct, wshift;
   unsigned *status;
   int spin_limit;
 };
 // One cooperative launch that meets between passes.  There are usually no
-// long segments, and then a launch for every pass was most of a call: in
-// segments of 64, a launch a pass / this, us: 2^16 int keys 37 / 22, 2^20
-// float64 71 / 34; with long segments, 2^19 int bimodal 80 / 71, 2^20 float64
-// log-normal 161 / 144.  In the larger tiles of longer vectors the passes
-// themselves ran 2-5 % slower here (2^23 float64 log-normal 652 / 683, with
-// tickets) and stay apart.
+// long segments, and then a launch for every pass was much of a call: in
+// segments of 64, a launch a pass / this, us: 2^16 int keys 37 / 22, 2^24 202 /
+// 181; 2^20 float64 71 / 34.  With long segments: 2^19 int bimodal 80 / 71,
+// 2^24 611 / 598; float64 log-normal 2^20 161 / 144, 2^23 651 / 623.
 // All CTAs are resident and take their tiles in increasing order, so a tile's
 // look-back waits only for tiles that are being ranked: no tickets, whose two
 // round trips a pass the meeting would not make up for.  None of a pass's
@@ -636,7 +616,13 @@ __global__ void __launch_bounds__(RK_BLOCK, GCVL_RK_MINB) k_rank_long(const __gr
         a.kout = (unsigned *)l.key[~q & 1];
         a.rank = l.rank; a.segbase = l.segbase; a.shift = 8 * (q - P);
         if (q < passes - 1) radix_tile<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS, ITEMS>(a, n, tile);
-        else radix_tile<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, ITEMS>(a, n, tile);
+        else if (ITEMS != RK_ITEMS_LARGE || l.direct)
+          radix_tile<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, ITEMS>(a, n, tile);
+        else if constexpr (ITEMS == RK_ITEMS_LARGE) {  // the pairs by window take the buffers this pass does not read
+          a.pidx = a.vout; a.ppos = a.kout;
+          a.wstate = l.state[(q + 1) % 3]; a.wshift = l.wshift;
+          radix_tile<unsigned, unsigned, false, IN_ARRAYS, OUT_WIN, ITEMS>(a, n, tile);
+        }
       }
       __syncthreads();
     }
@@ -889,28 +875,26 @@ __global__ void __launch_bounds__(RK_BLOCK) k_gather_gated(V *__restrict__ d, co
   }
 }
 
-template <class K, class V, bool AUX, int IN, int OUT, int ITEMS, bool DYN>
+template <class K, class V, bool AUX, int IN, int OUT, int ITEMS>
 void launch_pass_items(const PassArgs<K, V> &a) {
   constexpr size_t sm = pass_smem<K, V, AUX, ITEMS>();
   static bool attr = false;
   if (!attr) {
-    GCVL_CK(cudaFuncSetAttribute(k_radix_pass<K, V, AUX, IN, OUT, ITEMS, DYN>,
+    GCVL_CK(cudaFuncSetAttribute(k_radix_pass<K, V, AUX, IN, OUT, ITEMS>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     attr = true;
   }
-  int grid = ceil_div(a.n, RK_BLOCK * ITEMS);
-  if (DYN) grid = std::min(grid, st().sm_count * rk_minb<K, AUX>());
-  k_radix_pass<K, V, AUX, IN, OUT, ITEMS, DYN><<<grid, RK_BLOCK, sm, stream()>>>(a);
+  k_radix_pass<K, V, AUX, IN, OUT, ITEMS><<<ceil_div(a.n, RK_BLOCK * ITEMS), RK_BLOCK, sm, stream()>>>(a);
   launch_check("k_radix_pass");
 }
 inline int rk_tile(long n) {
   return RK_BLOCK * (n <= RK_TINY_MAX ? RK_ITEMS_TINY : n <= RK_SMALL_MAX ? RK_ITEMS_SMALL : RK_ITEMS_LARGE);
 }
-template <class K, class V, bool AUX, int IN, int OUT, bool DYN> void launch_pass(const PassArgs<K, V> &a) {
-  if (a.n > RK_SMALL_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_LARGE, DYN>(a);
-  else if constexpr (OUT != OUT_WIN && !DYN) {
-    if (a.n > RK_TINY_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_SMALL, DYN>(a);
-    else launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_TINY, DYN>(a);
+template <class K, class V, bool AUX, int IN, int OUT> void launch_pass(const PassArgs<K, V> &a) {
+  if (a.n > RK_SMALL_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_LARGE>(a);
+  else if constexpr (OUT != OUT_WIN) {
+    if (a.n > RK_TINY_MAX) launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_SMALL>(a);
+    else launch_pass_items<K, V, AUX, IN, OUT, RK_ITEMS_TINY>(a);
   }
 }
 template <class K, int ITEMS> void launch_long_items(LongArgs<K> l, int n) {
@@ -930,7 +914,8 @@ template <class K, int ITEMS> void launch_long_items(LongArgs<K> l, int n) {
   launch_check("k_rank_long");
 }
 template <class K> void launch_long(const LongArgs<K> &l, int n) {
-  if (n > RK_TINY_MAX) launch_long_items<K, RK_ITEMS_SMALL>(l, n);
+  if (n > RK_SMALL_MAX) launch_long_items<K, RK_ITEMS_LARGE>(l, n);
+  else if (n > RK_TINY_MAX) launch_long_items<K, RK_ITEMS_SMALL>(l, n);
   else launch_long_items<K, RK_ITEMS_TINY>(l, n);
 }
 static_assert(RK_SMALL_MAX <= RK_DIRECT_MAX, "windows only for large tiles");
@@ -1119,11 +1104,14 @@ template <bool DYN>
 __global__ void __launch_bounds__(RK_BLOCK) k_rank_scatter(int *__restrict__ rank, const unsigned *__restrict__ pidx,
                                                            const unsigned *__restrict__ ppos, int n, int wshift,
                                                            const unsigned long long *total,
-                                                           const unsigned *__restrict__ wstate, int tile_elems) {
+                                                           const unsigned *__restrict__ wstate, int tile_elems,
+                                                           const unsigned *status) {
   const unsigned *counts = nullptr;  // the last tile's inclusive window counts
   if constexpr (DYN) {
     const long t = (long)(unsigned)*(volatile const unsigned long long *)total;
     if (t == 0) return;
+    // a wait gave up: the pairs may be anything
+    if (*(volatile const unsigned *)status & DEV_TIMEOUT) return;
     counts = wstate + (t - 1) / tile_elems * 256;
   }
   for (long b = blockIdx.x; b * (RK_BLOCK * SC_ITEMS) < n; b += gridDim.x) {
@@ -1230,46 +1218,13 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
     l.rank = (int *)d; l.segbase = ls.base; l.hist = hist;
     for (int b = 0; b < 3; b++) l.state[b] = state[b];
     l.meet = counters + RK_MAXPASS;
-    l.total = total; l.seg_passes = seg_passes;
+    l.total = total; l.seg_passes = seg_passes; l.direct = direct; l.wshift = wshift;
     l.status = S.d_status; l.spin_limit = S.spin_limit;
-    if (n <= RK_SMALL_MAX) {
-      launch_long<K>(l, n);
-      return;
-    }
-    const int passes = key_passes + seg_passes;
-    for (int q = 0; q < passes; q++) {
-      const bool final = (q == passes - 1);
-      auto common = [&](auto &a) {
-        a.vin = l.idx[q & 1]; a.vout = l.idx[~q & 1];
-        a.hist = hist + q * 256; a.counter = counters + q;
-        a.state = state[q % 3]; a.clear = q > 0 && !final ? state[(q + 2) % 3] : nullptr;
-        a.total = total; a.n = n; a.status = S.d_status; a.spin_limit = S.spin_limit;
-      };
-      if (q < key_passes) {
-        PassArgs<K, unsigned> a{};
-        common(a);
-        a.kin = l.key[q & 1]; a.kout = l.key[~q & 1];
-        a.ain = l.aux[q & 1]; a.aout = l.aux[~q & 1];
-        a.shift = 8 * q;
-        launch_pass<K, unsigned, true, IN_ARRAYS, OUT_ARRAYS, true>(a);
-      } else {
-        // segment passes: the segment number is the key, indices ride along
-        PassArgs<unsigned, unsigned> a{};
-        common(a);
-        a.kin = q == key_passes ? aA : (const unsigned *)l.key[q & 1];
-        a.kout = (unsigned *)l.key[~q & 1];
-        a.segbase = ls.base; a.shift = 8 * (q - key_passes);
-        if (final) {  // the pairs by window take the buffers the last pass does not read
-          a.rank = (int *)d;
-          a.pidx = pidx = a.vout;
-          a.ppos = ppos = a.kout;
-          a.wstate = wstate = state[(q + 1) % 3]; a.wshift = wshift;
-        }
-        if (!final) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_ARRAYS, true>(a);
-        else if (direct) launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_RANK, true>(a);
-        else launch_pass<unsigned, unsigned, false, IN_ARRAYS, OUT_WIN, true>(a);
-      }
-    }
+    launch_long<K>(l, n);
+    const int last = key_passes + seg_passes - 1;
+    pidx = l.idx[~last & 1];
+    ppos = (unsigned *)l.key[~last & 1];
+    wstate = state[(last + 1) % 3];
   } else {
     // at least 16 keys a thread: every CTA adds its histograms to the vector's
     // with an atomic per bin (2^20 keys by 1216 CTAs 14.6 us, by 256 5)
@@ -1292,10 +1247,10 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
         a.ppos = ppos = (unsigned *)kB;
         a.wstate = state[(q + 1) % 3]; a.wshift = wshift;
       }
-      if (q == 0) launch_pass<K, unsigned, false, IN_SRC, OUT_ARRAYS, false>(a);
-      else if (!final) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_ARRAYS, false>(a);
-      else if (direct) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_RANK, false>(a);
-      else launch_pass<K, unsigned, false, IN_ARRAYS, OUT_WIN, false>(a);
+      if (q == 0) launch_pass<K, unsigned, false, IN_SRC, OUT_ARRAYS>(a);
+      else if (!final) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_ARRAYS>(a);
+      else if (direct) launch_pass<K, unsigned, false, IN_ARRAYS, OUT_RANK>(a);
+      else launch_pass<K, unsigned, false, IN_ARRAYS, OUT_WIN>(a);
       std::swap(kA, kB);
       std::swap(iA, iB);
     }
@@ -1304,10 +1259,10 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
   if (!direct) {
     if (seg)
       k_rank_scatter<true><<<sc_grid(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, total, wstate,
-                                                                  rk_tile(n));
+                                                                  rk_tile(n), S.d_status);
     else
       k_rank_scatter<false><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, nullptr, nullptr,
-                                                                     rk_tile(n));
+                                                                     rk_tile(n), nullptr);
     launch_check("k_rank_scatter");
   }
 }

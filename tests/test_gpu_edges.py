@@ -95,7 +95,7 @@ def test_rank_long_segments_by_window(gpu, oracle, name, n):
 @pytest.mark.parametrize("name", ["rkd_lez", "rku_led"])
 def test_rank_long_segments_captured(gpu, oracle, name, n):
     """The passes over the long segments inside a CUDA graph, replayed on other keys, in each of their tile sizes
-    (up to 2^20 elements in one launch that meets between passes); then the same call outside it."""
+    (one launch that meets between passes); then the same call outside it."""
     r = W.rng(n + 3)
     lens = np.array([2049, 0, 7, n - 2056], dtype=np.int32)
     if n == 4097:
