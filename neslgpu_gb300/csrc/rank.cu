@@ -36,6 +36,7 @@
 // window split below) and share the window scatter.
 #include "gcvl.cuh"
 #include "rank.cuh"
+#include "rank_warp.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -327,60 +328,13 @@ __device__ __forceinline__ void radix_tile(const PassArgs<K, V> &a, const int n,
     }
   }
 
-  // Rank within each warp's elements: (rank << 8) | digit.  An item's peers
-  // (the lanes with its digit) come from a lane mask per digit in shared
-  // memory, where the tile is reordered later: every lane sets its bit, reads
-  // the mask back, and the first peer counts for all and clears it; G items
-  // at a time with masks of their own, so that their accesses are in flight
-  // together.  Eight ballots an item (four ALU instructions a bit) kept the
-  // ALU busy and the shared-memory pipe idle: a pass over 2^26 keys 406 us,
-  // now 370 us with the shared-memory pipe 77 % busy.  Ballots for one, two
-  // or three of every five items changed nothing or lost; counting without
-  // masks and ordering the lanes that share a digit afterwards took 4 % more.
-  // An item whose lanes all hold one digit skips the masks: 32 adds to one
-  // word take turns (2^25 keys of two values 1217 -> 961 us, 1183 with the
-  // ballots; random keys pay 1.5 %).
-  unsigned *cnt = s_cnt + warp * 256;
-  const unsigned lt = (1u << lane) - 1u;
-  constexpr int G = RK_ITEMS / 4;
-  unsigned *mask = (unsigned *)s_kout + warp * 256;  // [G][RK_WARPS][256]
-  static_assert((size_t)G * RK_WARPS * 256 * 4 <= (size_t)RK_TILE * (sizeof(K) + sizeof(V)) && RK_ITEMS % G == 0,
+  // the ranks within each warp's elements, by lane masks where the tile is reordered later
+  constexpr int G = RK_ITEMS / 4;  // [G][RK_WARPS][256] masks
+  static_assert((size_t)G * RK_WARPS * 256 * 4 <= (size_t)RK_TILE * (sizeof(K) + sizeof(V)),
                 "the masks fit where the tile is reordered");
   unsigned wr[RK_ITEMS];
-#pragma unroll
-  for (int c0 = 0; c0 < RK_ITEMS; c0 += G) {
-    unsigned m[G];
-    bool one[G];  // all lanes hold the same digit
-#pragma unroll
-    for (int u = 0; u < G; u++) {
-      const unsigned d = (unsigned)(kr[c0 + u] >> a.shift) & 255u;
-      one[u] = __all_sync(0xffffffffu, d == shfl_idx(d, 0));
-      if (!one[u]) atomicOr(mask + u * RK_WARPS * 256 + d, 1u << lane);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < G; u++) {
-      m[u] = 0xffffffffu;
-      if (!one[u]) m[u] = mask[u * RK_WARPS * 256 + ((unsigned)(kr[c0 + u] >> a.shift) & 255u)];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < G; u++) {
-      const unsigned d = (unsigned)(kr[c0 + u] >> a.shift) & 255u;
-      unsigned r = 0;
-      if ((m[u] & lt) == 0) {
-        r = atomicAdd(cnt + d, (unsigned)__popc(m[u]));
-        mask[u * RK_WARPS * 256 + d] = 0;
-      }
-      wr[c0 + u] = r;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < G; u++) {
-      const unsigned d = (unsigned)(kr[c0 + u] >> a.shift) & 255u;
-      wr[c0 + u] = ((shfl_idx(wr[c0 + u], __ffs(m[u]) - 1) + __popc(m[u] & lt)) << 8) | d;
-    }
-  }
+  warp_digit_ranks<RK_ITEMS, G>(wr, kr, a.shift, s_cnt + warp * 256, (unsigned *)s_kout + warp * 256, RK_WARPS * 256,
+                                lane);
   __syncthreads();
 
   // per digit: tile count, per-warp exclusive offsets
