@@ -224,12 +224,24 @@ template <class K, class V> struct PassArgs {
   int wshift;                         // OUT_WIN: window of v = v >> wshift
   unsigned *counter;
   int n, shift;
-  unsigned *status;
+  unsigned *status, *gave_up;         // gave_up: marked RK_STOP when a wait of this pass runs out
   int spin_limit;
 };
 
 template <class K, class V, bool AUX, int ITEMS> constexpr size_t pass_smem() {
   return (size_t)RK_BLOCK * ITEMS * (sizeof(K) + sizeof(V) + (AUX ? 4 : 0)) + RK_WARPS * 256 * 4 + 256 * 4 + 256 * 8;
+}
+
+// A wait of this call gave up: noted for the host, and in a word of the call's
+// own.  What a pass writes after that stays inside its outputs (a prefix only
+// comes out too small), but places are left unwritten, so no later pass of the
+// call may take its output for indices.  The word is cleared with the call's
+// tickets; the status word stays set until the host reads it, and the calls
+// that come before then are carried out.
+constexpr unsigned RK_STOP = 0x80000000u;
+__device__ __forceinline__ void rk_give_up(unsigned *status, unsigned *gave_up) {
+  atomicOr(status, DEV_TIMEOUT);
+  atomicOr(gave_up, RK_STOP);
 }
 
 // Publish this tile's count of one bin (digit or window), then look back for
@@ -241,7 +253,7 @@ template <class K, class V, bool AUX, int ITEMS> constexpr size_t pass_smem() {
 // relaxed loads suffice and all RK_LB are in flight together; a warp's loads
 // of one predecessor are one 128-byte line.
 __device__ __forceinline__ unsigned bin_lookback(unsigned *state, int tile, int bin, unsigned tot,
-                                                 unsigned *status, int spin_limit) {
+                                                 unsigned *status, unsigned *gave_up, int spin_limit) {
   unsigned *stw = state + (long)tile * 256 + bin;
   if (tile == 0) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(stw), "r"(RK_INC | tot) : "memory");
@@ -264,7 +276,7 @@ __device__ __forceinline__ unsigned bin_lookback(unsigned *state, int tile, int 
       if (done) break;
       int it = 0;
       while (w[j] == 0) {
-        if (++it >= spin_limit) { atomicOr(status, DEV_TIMEOUT); w[j] = RK_INC; break; }
+        if (++it >= spin_limit) { rk_give_up(status, gave_up); w[j] = RK_INC; break; }
         __nanosleep(32);
         asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(w[j]) : "l"(state + (t0 - j) * 256 + bin) : "memory");
       }
@@ -347,7 +359,7 @@ __device__ __forceinline__ void radix_tile(const PassArgs<K, V> &a, const int n,
     s_cnt[w * 256 + dd] = tot;
     tot += c;
   }
-  const unsigned prefix = bin_lookback(a.state, tile, dd, tot, a.status, a.spin_limit);
+  const unsigned prefix = bin_lookback(a.state, tile, dd, tot, a.status, a.gave_up, a.spin_limit);
   // exclusive scans over the digits of the tile's counts -> tile offsets,
   // and of the vector's counts -> digit starts
   {
@@ -404,7 +416,7 @@ __device__ __forceinline__ void radix_tile(const PassArgs<K, V> &a, const int n,
     }
     __syncthreads();
     const unsigned wtot = s_wc[tid];
-    const unsigned wprefix = bin_lookback(a.wstate, tile, tid, wtot, a.status, a.spin_limit);
+    const unsigned wprefix = bin_lookback(a.wstate, tile, tid, wtot, a.status, a.gave_up, a.spin_limit);
     {
       unsigned incl = wtot;
 #pragma unroll
@@ -480,12 +492,19 @@ __device__ __forceinline__ void radix_tile(const PassArgs<K, V> &a, const int n,
   }
 }
 
-// One tile per CTA, taken in ticket order.
+// One tile per CTA, taken in ticket order.  The word that a pass's waits mark
+// when they give up is the next pass's ticket counter: that pass's tickets
+// then are no tiles, and it marks the one after it and writes nothing.  (A
+// word apart, read by every CTA, took 1.4 % of a rank of 2^26 keys.)
 template <class K, class V, bool AUX, int IN, int OUT, int ITEMS>
 __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(PassArgs<K, V> a) {
   __shared__ unsigned s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(a.counter, 1u);
+  if (threadIdx.x == 0) {
+    s_tile = atomicAdd(a.counter, 1u);
+    if (s_tile & RK_STOP) atomicOr(a.gave_up, RK_STOP);
+  }
   __syncthreads();
+  if (s_tile & RK_STOP) return;
   radix_tile<K, V, AUX, IN, OUT, ITEMS>(a, a.n, (int)s_tile);
 }
 
@@ -493,8 +512,9 @@ __global__ void __launch_bounds__(RK_BLOCK, rk_minb<K, AUX>()) k_radix_pass(Pass
 // what any of them stored before, all may load afterwards.  Returns the
 // CTA's number, read from memory after the wait, so that loads whose address
 // comes from it cannot be moved ahead; negative when the bounded wait, or any
-// wait before it, gave up (the next pass would follow indices nobody wrote).
-__device__ __forceinline__ int rk_meet(unsigned *count, unsigned arrivals, unsigned *status, int limit) {
+// wait of the call before it, gave up (the next pass would follow indices nobody wrote).
+__device__ __forceinline__ int rk_meet(unsigned *count, unsigned arrivals, unsigned *status, unsigned *gave_up,
+                                       int limit) {
   __shared__ volatile int s_cta;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -502,11 +522,11 @@ __device__ __forceinline__ int rk_meet(unsigned *count, unsigned arrivals, unsig
     __threadfence();
     atomicAdd(count, 1u);
     while (*(volatile unsigned *)count < arrivals) {
-      if (++it >= limit) { ok = 0; atomicOr(status, DEV_TIMEOUT); break; }
+      if (++it >= limit) { ok = 0; rk_give_up(status, gave_up); break; }
       if (it > 64) __nanosleep(32);
     }
     __threadfence();
-    s_cta = ok && !(*(volatile unsigned *)status & DEV_TIMEOUT) ? (int)blockIdx.x : -1;
+    s_cta = ok && !*(volatile unsigned *)gave_up ? (int)blockIdx.x : -1;
   }
   __syncthreads();
   return s_cta;
@@ -522,7 +542,7 @@ template <class K> struct LongArgs {
   unsigned *state[3], *meet;
   const unsigned long long *total;
   int seg_passes, direct, wshift;
-  unsigned *status;
+  unsigned *status, *gave_up;
   int spin_limit;
 };
 // One cooperative launch that meets between passes.  There are usually no
@@ -548,12 +568,12 @@ __global__ void __launch_bounds__(RK_BLOCK, GCVL_RK_MINB) k_rank_long(const __gr
     a.hist = l.hist + q * 256;
     a.state = l.state[q % 3];
     a.clear = q > 0 && q < passes - 1 ? l.state[(q + 2) % 3] : nullptr;
-    a.status = l.status; a.spin_limit = l.spin_limit;
+    a.status = l.status; a.gave_up = l.gave_up; a.spin_limit = l.spin_limit;
   };
   int first = blockIdx.x;
 #pragma unroll 1
   for (int q = 0; q < passes; q++) {
-    if (q > 0 && (first = rk_meet(l.meet, (unsigned)(q * ctas), l.status, l.spin_limit)) < 0) return;
+    if (q > 0 && (first = rk_meet(l.meet, (unsigned)(q * ctas), l.status, l.gave_up, l.spin_limit)) < 0) return;
 #pragma unroll 1
     for (int tile = first; tile < tiles; tile += ctas) {
       if (q < P) {
@@ -1053,19 +1073,21 @@ template void scatter_partitioned<unsigned long long>(unsigned long long *, cons
 // grouped by window of the index: window w's pairs lie from slot w << wshift
 // on, as many as the last pass counted (all the window's indices when the
 // vector was ranked whole).  One CTA per 2048 slots, as k_window_scatter;
-// DYN (long segments, usually none): a resident grid.
+// DYN (long segments, usually none): a resident grid.  After a wait of the
+// passes gave up the pairs may be anything: DYN, whose counts may be missing
+// too, writes nothing, and otherwise an index is looked at before it is
+// followed (10 us of 340 at 2^26 keys; asking the word in every CTA took 20).
 template <bool DYN>
 __global__ void __launch_bounds__(RK_BLOCK) k_rank_scatter(int *__restrict__ rank, const unsigned *__restrict__ pidx,
                                                            const unsigned *__restrict__ ppos, int n, int wshift,
                                                            const unsigned long long *total,
                                                            const unsigned *__restrict__ wstate, int tile_elems,
-                                                           const unsigned *status) {
+                                                           const unsigned *gave_up) {
   const unsigned *counts = nullptr;  // the last tile's inclusive window counts
   if constexpr (DYN) {
     const long t = (long)(unsigned)*(volatile const unsigned long long *)total;
     if (t == 0) return;
-    // a wait gave up: the pairs may be anything
-    if (*(volatile const unsigned *)status & DEV_TIMEOUT) return;
+    if (*(const volatile unsigned *)gave_up) return;
     counts = wstate + (t - 1) / tile_elems * 256;
   }
   for (long b = blockIdx.x; b * (RK_BLOCK * SC_ITEMS) < n; b += gridDim.x) {
@@ -1081,7 +1103,7 @@ __global__ void __launch_bounds__(RK_BLOCK) k_rank_scatter(int *__restrict__ ran
     }
 #pragma unroll
     for (int u = 0; u < SC_ITEMS; u++)
-      if (ok[u]) rank[k[u]] = (int)v[u];
+      if (ok[u] && k[u] < (unsigned)n) rank[k[u]] = (int)v[u];
     if (!DYN) return;
   }
 }
@@ -1099,7 +1121,7 @@ inline RankLayout rank_layout(int n, int is_double, int seg) {
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += align_up(bytes, 256); return at; };
   L.hist = take(RK_MAXPASS * 256 * 4);  // these three are cleared together
-  L.counter = take((RK_MAXPASS + 1) * 4);  // tickets, and the long segments' meetings
+  L.counter = take((RK_MAXPASS + 2) * 4);  // tickets, the long segments' meetings, and whether a wait gave up
   L.lsum = take(8);
   L.state = take(rk_state_bytes(n) * 3);
   L.key_a = take((size_t)n * ks);
@@ -1148,7 +1170,7 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
   const int key_passes = (int)sizeof(K);
   const bool direct = n <= RK_DIRECT_MAX;
   const int wshift = window_shift(n);
-  unsigned *pidx = nullptr, *ppos = nullptr, *wstate = nullptr;
+  unsigned *pidx = nullptr, *ppos = nullptr, *wstate = nullptr, *gave_up = nullptr;
   const unsigned long long *total = nullptr;
   if (seg) {
     LongSegs ls;
@@ -1173,7 +1195,7 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
     for (int b = 0; b < 3; b++) l.state[b] = state[b];
     l.meet = counters + RK_MAXPASS;
     l.total = total; l.seg_passes = seg_passes; l.direct = direct; l.wshift = wshift;
-    l.status = S.d_status; l.spin_limit = S.spin_limit;
+    l.status = S.d_status; l.gave_up = gave_up = counters + RK_MAXPASS + 1; l.spin_limit = S.spin_limit;
     launch_long<K>(l, n);
     const int last = key_passes + seg_passes - 1;
     pidx = l.idx[~last & 1];
@@ -1194,7 +1216,7 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
       a.src = s; a.up = up; a.shift = 8 * q;
       a.hist = hist + q * 256; a.counter = counters + q;
       a.state = state[q % 3]; a.clear = q > 0 && !final ? state[(q + 2) % 3] : nullptr;
-      a.n = n; a.status = S.d_status; a.spin_limit = S.spin_limit;
+      a.n = n; a.status = S.d_status; a.gave_up = counters + q + 1; a.spin_limit = S.spin_limit;
       if (final) {  // the pairs by window take the buffers the last pass does not read
         a.rank = (int *)d;
         a.pidx = pidx = iB;
@@ -1213,7 +1235,7 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
   if (!direct) {
     if (seg)
       k_rank_scatter<true><<<sc_grid(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, total, wstate,
-                                                                  rk_tile(n), S.d_status);
+                                                                  rk_tile(n), gave_up);
     else
       k_rank_scatter<false><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, nullptr, nullptr,
                                                                      rk_tile(n), nullptr);

@@ -64,3 +64,68 @@ def test_injected_spin_limit_never_hangs(gpu):
         c.gcvl_set_spin_limit(old)
         c.gcvl_clear_error()
     compare("sum", ops.scan_e(gpu, "add_sed", x, one), want, S)
+
+
+def _rank_case(r, name, n):
+    """Keys and, for a segmented rank, lengths among which are some that the digit passes take."""
+    x = W.float64_normal(r, n) if name[-1] == "d" else W.int32_uniform(r, n)
+    if name[5] == "u":
+        return x, None
+    return x, np.array([5, n // 2, 0, 1, n - n // 2 - 6], dtype=np.int32)
+
+
+def _rank(R, name, x, lens):
+    return ops.rank_u(R, name, x) if lens is None else ops.rank_e(R, name, x, lens)
+
+
+# sizes of the digit passes' three tile sizes; past 2^23 the ranks go through windows
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [200_003, 1_000_003, (1 << 23) + 5])
+@pytest.mark.parametrize("name", ["rku_luz", "rkd_lud", "rkd_lez", "rku_led"])
+def test_ranks_whose_waits_run_out(gpu, oracle, name, n):
+    """With the wait limit forced to 1 the digit passes' look-back and meetings give up: the ranks are right, or
+    flagged and then nothing is written past their vector; the next call is right again."""
+    c = gpu.cvl
+    x, lens = _rank_case(W.rng(n), name, n)
+    want = _rank(oracle, name, x, lens)
+    old = c.gcvl_get_spin_limit()
+    k, d = gpu.vec(x, name[-1]), gpu.vec(np.full(n + 4096, -1, dtype=np.int32), "z")
+    sd, sizes = (None, (n,)) if lens is None else (gpu.segd(lens)[0], (n, lens.size))
+    scr = gpu.units(gpu.fn(name + "_scratch")(*sizes))
+    assert c.gcvl_sync() == 0
+    try:
+        c.gcvl_set_spin_limit(1)
+        gpu.fn(name)(d.ptr, k.ptr, *([sd.ptr] if sd else []), *sizes, scr.ptr)
+        code = c.gcvl_sync()
+        got = d.numpy(n + 4096)
+        assert code in (0, 3)
+        assert np.all(got[n:] == -1)
+        if code == 0:
+            assert np.array_equal(got[:n], want)
+    finally:
+        c.gcvl_set_spin_limit(old)
+        c.gcvl_clear_error()
+    assert np.array_equal(_rank(gpu, name, x, lens), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [300_000, (1 << 23) + 5])
+@pytest.mark.parametrize("name", ["rku_lez", "rkd_led", "rku_luz"])
+def test_ranks_after_an_earlier_call_gave_up(gpu, oracle, name, n):
+    """A wait that gave up stays noted until gcvl_sync; the calls before that are carried out all the same."""
+    c = gpu.cvl
+    old = c.gcvl_get_spin_limit()
+    r = W.rng(n + 1)
+    y = W.float64_normal(r, 1 << 22)
+    x, lens = _rank_case(r, name, n)
+    R = ops.DeviceRunner(c, checked=False)
+    try:
+        c.gcvl_set_spin_limit(1)
+        ops.scan_e(R, "add_sed", y, np.array([y.size], dtype=np.int32))
+        c.gcvl_set_spin_limit(old)
+        got = _rank(R, name, x, lens)
+        assert c.gcvl_sync() in (0, 3)
+    finally:
+        c.gcvl_set_spin_limit(old)
+        c.gcvl_clear_error()
+    assert np.array_equal(got, _rank(oracle, name, x, lens))
