@@ -604,10 +604,11 @@ __global__ void __launch_bounds__(RK_BLOCK, GCVL_RK_MINB) k_rank_long(const __gr
 }
 
 // d[key[i]] = val[i], streaming over pairs that a partition pass grouped by
-// output window
+// output window.  A key past n_d is followed nowhere: after a wait that gave
+// up some pairs are unwritten.
 template <class V>
 __global__ void __launch_bounds__(RK_BLOCK) k_window_scatter(V *__restrict__ d, const unsigned *__restrict__ key,
-                                                             const V *__restrict__ val, long n,
+                                                             const V *__restrict__ val, long n, unsigned n_d,
                                                              const unsigned *__restrict__ gate) {
   // one CTA per 2048 pairs, not a grid-stride loop: CTAs dispatched in
   // order keep the writes within a few windows of the output at a time
@@ -624,7 +625,7 @@ __global__ void __launch_bounds__(RK_BLOCK) k_window_scatter(V *__restrict__ d, 
 #pragma unroll
   for (int u = 0; u < SC_ITEMS; u++) {
     const long i = i0 + (long)u * RK_BLOCK;
-    if (i < n) d[k[u]] = v[u];
+    if (i < n && k[u] < n_d) d[k[u]] = v[u];
   }
 }
 
@@ -752,6 +753,8 @@ __global__ void __launch_bounds__(RK_BLOCK) k_window_split(const unsigned *__res
   __syncthreads();
   // the windows' first slots within the tile: exclusive scan over the bins
   const unsigned tot = s_cnt[tid];
+  // a scan whose wait gave up can leave any slot here: the tile's keys stay inside the n
+  if (tid < nw) s_base[tid] = min(s_base[tid], (unsigned)n - tot);
   unsigned incl = tot;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -995,7 +998,7 @@ void scatter_partitioned(V *d, const V *s, const int *idx, int n, int n_d, vec_p
   k_window_split<false, V, true><<<tiles, RK_BLOCK, smem, S.stream>>>((const unsigned *)idx, n, shift, wbits, counts,
                                                                       unsorted, kout, nullptr, s, vout);
   launch_check("k_window_split");
-  k_window_scatter<V><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>(d, kout, vout, n, unsorted);
+  k_window_scatter<V><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>(d, kout, vout, n, (unsigned)n_d, unsorted);
   launch_check("k_window_scatter");
 }
 

@@ -129,3 +129,40 @@ def test_ranks_after_an_earlier_call_gave_up(gpu, oracle, name, n):
         c.gcvl_set_spin_limit(old)
         c.gcvl_clear_error()
     assert np.array_equal(got, _rank(oracle, name, x, lens))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [(1 << 23) + 5, (1 << 25) + 3])
+@pytest.mark.parametrize("name", ["smp_puz", "bck_puz", "smp_pud", "bck_pud"])
+def test_random_permutes_whose_waits_run_out(gpu, name, n):
+    """With the wait limit forced to 1 the scan of the window split's counts may give up: the result is right, or
+    flagged and then nothing is written past its vector; the next call is right again."""
+    c = gpu.cvl
+    r = W.rng(n)
+    x = W.float64_normal(r, n) if name[-1] == "d" else W.int32_uniform(r, n)
+    perm = r.permutation(n).astype(np.int32)
+    want = np.empty_like(x)
+    if name[0] == "s":
+        want[perm] = x
+    else:
+        want = x[perm]
+    sizes = (n,) if name[0] == "s" else (n, n)
+    guard = x[:4096]
+    s, p, d = gpu.vec(x, name[-1]), gpu.vec(perm, "z"), gpu.vec(np.concatenate([x, guard]), name[-1])
+    scr = gpu.units(gpu.fn(name + "_scratch")(*sizes))
+    old = c.gcvl_get_spin_limit()
+    assert c.gcvl_sync() == 0
+    try:
+        for limit in (1, old):
+            c.gcvl_set_spin_limit(limit)
+            gpu.fn(name)(d.ptr, s.ptr, p.ptr, *sizes, scr.ptr)
+            code = c.gcvl_sync()
+            got = d.numpy(n + guard.size)
+            assert code in ((0, 3) if limit == 1 else (0,))
+            assert np.array_equal(got[n:], guard)
+            if code == 0:
+                assert np.array_equal(got[:n], want)
+            c.gcvl_clear_error()
+    finally:
+        c.gcvl_set_spin_limit(old)
+        c.gcvl_clear_error()
