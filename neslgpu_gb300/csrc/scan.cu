@@ -1911,7 +1911,7 @@ __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_o
       while (hi - lo > 1) {
         const int step = (hi - lo + 31) / 32, at = min(lo + lane * step, hi);
         const unsigned below = __ballot_sync(0xffffffffu, at < hi && off_at(at) <= e);
-        const int k = 31 - __clz(below);  // lane 0 probes lo itself
+        const int k = max(31 - __clz(below), 0);  // lane 0 probes lo itself; offsets of a scan that gave up need not ascend
         hi = min(lo + (k + 1) * step, hi);
         lo += k * step;
       }
@@ -1925,7 +1925,7 @@ __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_o
       unsigned bit = 0;
       if (s <= last) {
         const int o = off_at(s);
-        if (o >= e0 && off_at(s + 1) > o) {  // a non-empty segment that starts here
+        if (o >= e0 && o < e1 && off_at(s + 1) > o) {  // a non-empty segment that starts here
           const int r = (int)(o - e0);
           word = r >> 5;
           bit = 1u << (r & 31);

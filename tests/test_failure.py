@@ -166,3 +166,43 @@ def test_random_permutes_whose_waits_run_out(gpu, name, n):
     finally:
         c.gcvl_set_spin_limit(old)
         c.gcvl_clear_error()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,m", [(1 << 20, 300_001), (1 << 25, (1 << 22) + 3), (3_000_000, 1 << 20)])
+def test_descriptors_whose_waits_run_out(gpu, oracle, n, m):
+    """With the wait limit forced to 1 the scan of the lengths gives up and leaves offsets that do not ascend: nothing
+    is written past the descriptor, and the next call is right again.  Lengths apart and in place."""
+    c = gpu.cvl
+    r = W.rng(m)
+    lens = np.diff(np.concatenate([[0], np.sort(r.integers(0, n + 1, size=m - 1)), [n]])).astype(np.int32)
+    units, guard = c.siz_fos(n, m), np.arange(4096, dtype=np.int32)
+    old = c.gcvl_get_spin_limit()
+    scr = gpu.units(c.mke_fov_scratch(n, m))
+    x = W.int32_uniform(r, n)
+    want = ops.reduce_e(oracle, "max_rez", x, lens)
+    xv, y = gpu.vec(x, "z"), gpu.out(m, "z")
+    rscr = gpu.units(gpu.fn("max_rez_scratch")(n, m))
+    for in_place in (False, True):
+        sd = gpu.vec(np.zeros(2 * units + guard.size, dtype=np.int32), "z")
+        lv = gpu.vec(lens, "z")
+        tail = c.add_fov(sd.ptr, units)
+        try:
+            for limit in (1, old):
+                c.c2v_fuz(tail, guard.ctypes.data, guard.size, None)
+                if in_place:
+                    c.c2v_fuz(sd.ptr, lens.ctypes.data, m, None)
+                assert c.gcvl_sync() == 0
+                c.gcvl_set_spin_limit(limit)
+                c.mke_fov(sd.ptr, sd.ptr if in_place else lv.ptr, n, m, scr.ptr)
+                code = c.gcvl_sync()
+                assert code in ((0, 3) if limit == 1 else (0,))
+                c.gcvl_clear_error()
+                got = np.empty(guard.size, dtype=np.int32)
+                c.v2c_fuz(got.ctypes.data, tail, guard.size, None)
+                assert np.array_equal(got, guard)
+        finally:
+            c.gcvl_set_spin_limit(old)
+            c.gcvl_clear_error()
+        gpu.fn("max_rez")(y.ptr, xv.ptr, sd.ptr, n, m, rscr.ptr)
+        assert np.array_equal(gpu.get(y, m), want)
