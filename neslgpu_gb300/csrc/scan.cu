@@ -1845,7 +1845,19 @@ void seg_scan(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, const cha
 // launch (at most two ranges per SM).
 // Few ranges take 512 threads each, more than two per SM 256 (2^18 one-element
 // segments 21 us against 29; 2^25 elements in segments of 64 29 against 22).
-constexpr int SD_RANGE = 256 * 32, SD_GRAN = SD_RANGE / kGranule, SD_SMALL = 4096;
+// Segments a CTA walks before it searches instead: a range with that many is
+// mostly empty segments, and SD_RANGE searches bound what it takes however
+// many there are.  With two segments per element (four where the ranges fill
+// the GPU and the searches miss L2) most are certainly empty, and the searches
+// are spread over more CTAs (k_segdes_sparse).  Walks alone / now / a cleared
+// bitmap, a search per granule and an atomic per head, us: 2^20 elements with
+// 2^20 empty segments in one place 783 / 30 / 29, 2^25 with 2^22 6329 / 57 / 49;
+// 8000 elements in 2^22 segments 3478 / 36 / 50, 2^16 in 2^20 150 / 21 / 34;
+// 2^22 in 2^23 94 / 95 / 91.
+constexpr int SD_RANGE = 256 * 32, SD_GRAN = SD_RANGE / kGranule, SD_SMALL = 4096, SD_SEARCH = 8;
+constexpr int sd_walk(int block) { return block == 512 ? 4 * SD_RANGE : 16 * SD_RANGE; }
+constexpr long SD_SPARSE = 2;
+static_assert(SD_RANGE % (SD_SEARCH * 512) == 0, "whole groups of searches");
 static_assert(SD_RANGE == 32 * 256, "the bitmap is padded to whole ranges");
 template <bool OFFS, int SD_BLOCK>
 __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_out, int *off, int *__restrict__ gran,
@@ -1919,6 +1931,36 @@ __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_o
     }
     __syncthreads();
     const int first = s_ends[0], last = s_ends[1];
+    if (!OFFS && last - first >= sd_walk(SD_BLOCK)) {
+      // mostly empty segments: the segment of every element by a search
+      // instead of every segment's element, SD_SEARCH searches of a lane in flight
+      int top = 1;
+      while (2 * top <= last - first) top *= 2;
+      const long g0 = e0 / kGranule;
+#pragma unroll 1
+      for (int b = warp * 32; b < SD_RANGE; b += SD_SEARCH * SD_BLOCK) {
+        int at[SD_SEARCH];
+#pragma unroll
+        for (int u = 0; u < SD_SEARCH; u++) at[u] = first;
+#pragma unroll 1
+        for (int step = top; step; step >>= 1) {
+#pragma unroll
+          for (int u = 0; u < SD_SEARCH; u++) {
+            const int to = at[u] + step;
+            if (to <= last && off_at(to) <= e0 + b + u * SD_BLOCK + lane) at[u] = to;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < SD_SEARCH; u++) {
+          const int r = b + u * SD_BLOCK + lane;  // the element's place in the range
+          const unsigned w = __ballot_sync(0xffffffffu, e0 + r < e1 && off_at(at[u]) == e0 + r);
+          if (lane == 0) bits[(e0 + r) >> 5] = w;
+          if (r % kGranule == 0 && e0 + r < e1) gran[g0 + r / kGranule] = at[u];
+        }
+      }
+      if (blockIdx.x == gridDim.x - 1 && tid == 0) gran[ng] = m;
+      return;
+    }
     for (int s0 = first + warp * 32; s0 <= last; s0 += SD_BLOCK) {
       const int s = s0 + lane;
       int word = -1, g = -1;
@@ -1968,6 +2010,25 @@ __global__ void __launch_bounds__(SD_BLOCK) k_segdes(const int *lens, int *len_o
   if (blockIdx.x == gridDim.x - 1 && tid == 0) gran[ng] = m;
 }
 
+// The tables where most segments are certainly empty: an element a thread,
+// which searches the segment that holds it, so that a vector of few elements
+// and many segments is spread over the GPU too.
+constexpr int SD_EBLOCK = 256;
+__global__ void __launch_bounds__(SD_EBLOCK) k_segdes_sparse(const int *__restrict__ off, int *__restrict__ gran,
+                                                             unsigned *__restrict__ bits, int n, int m) {
+  const long e = (long)blockIdx.x * SD_EBLOCK + threadIdx.x;
+  int lo = 0, hi = m - 1;
+  if (e < n)
+    while (lo < hi) {
+      const int mid = lo + (hi - lo + 1) / 2;
+      if (__ldg(off + mid) <= e) lo = mid; else hi = mid - 1;
+    }
+  const unsigned w = __ballot_sync(0xffffffffu, e < n && __ldg(off + lo) == e);
+  if ((threadIdx.x & 31) == 0) bits[e >> 5] = w;
+  if (e < n && e % kGranule == 0) gran[e / kGranule] = lo;
+  if (e == 0) gran[((long)n + kGranule - 1) / kGranule] = m;
+}
+
 void make_segdes(vec_p sd, vec_p l, int n, int m, vec_p scratch) {
   ensure_init();
   State &S = st();
@@ -1995,8 +2056,11 @@ void make_segdes(vec_p sd, vec_p l, int n, int m, vec_p scratch) {
   } else {
     run_scan<AddZ, M_OFFSETS, false>(off, (const int *)l, len, nullptr, m, 1, scratch, false, "mke_fov");
   }
-  if (few) k_segdes<false, 512><<<ranges, 512, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
-  else k_segdes<false, 256><<<ranges, 256, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
+  if (m >= (few ? SD_SPARSE : 2 * SD_SPARSE) * n)
+    k_segdes_sparse<<<ranges * (SD_RANGE / SD_EBLOCK), SD_EBLOCK, 0, S.stream>>>(off, gran, bits, n, m);
+  else if (few) k_segdes<false, 512><<<ranges, 512, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
+  else
+    k_segdes<false, 256><<<ranges, 256, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
   launch_check("mke_fov");
 }
 

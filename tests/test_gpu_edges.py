@@ -330,3 +330,25 @@ def test_float_sums_of_even_segments(gpu, oracle, mean):
     mag = np.add.reduceat(np.abs(x), np.arange(m) * mean)
     g, o = ops.reduce_e(gpu, "add_red", x, lens), ops.reduce_e(oracle, "add_red", x, lens)
     assert np.all(np.abs(g - o) <= 1e-12 * mag)
+
+
+@pytest.mark.parametrize("where", ["spread", "one place", "end", "start"])
+@pytest.mark.parametrize("n,m", [(1, 5000), (63, 8193), (4097, 8193), (4097, 8194), (4097, 8195), (8192 * 3 + 5, 40_000),
+                                 (50_000, 99_999), (50_000, 100_000), (50_000, 300_000), (3_000_001, 1_200_000)])
+def test_descriptors_of_mostly_empty_segments(gpu, oracle, n, m, where):
+    """Either side of two segments per element, from which every element searches its segment, and of the
+    segments that a CTA walks over 8192 elements (32768, and 131072 beyond two ranges per SM)."""
+    r = W.rng(n + m)
+    lens = np.zeros(m, dtype=np.int32)
+    if where == "spread":
+        lens = np.diff(np.concatenate([[0], np.sort(r.integers(0, n + 1, size=m - 1)), [n]])).astype(np.int32)
+    else:  # the elements in few segments, the others empty in one place
+        k = min(n, 20)
+        cut = np.diff(np.concatenate([[0], np.sort(r.choice(np.arange(1, n), size=k - 1, replace=False)), [n]])) if k > 1 else [n]
+        at = {"one place": k // 2, "end": k, "start": 0}[where]
+        lens[:at], lens[m - (k - at):] = cut[:at], cut[at:]
+    x, v = W.int32_uniform(r, n), np.arange(m, dtype=np.int32)
+    for R in (gpu, oracle):
+        R.got = [ops.scan_e(R, "add_sez", x, lens), ops.reduce_e(R, "max_rez", x, lens), ops.dis_e(R, "dis_vez", v, lens)]
+    for a, b in zip(gpu.got, oracle.got):
+        assert np.array_equal(a, b)
