@@ -372,6 +372,13 @@ template <int ITEMS> struct Engine<AddD, ITEMS> {
 #define GCVL_RED_CHAIN_MEAN 128
 #endif
 constexpr long RED_CHAIN_MEAN = GCVL_RED_CHAIN_MEAN;
+// Items of a folded row that are added in FP64 instead: a row's fixed point
+// cuts every item at the unit of its largest, so it loses up to a unit an item.
+// All 16 in fixed point raised the mean error of long sums of exponential
+// values from 1.6 to 1.8 units in the last place, and where the last two
+// items are by far the largest from 0.6 to 6; the headline step of 2^28
+// elements takes 1492 us this way, 1483 that.
+constexpr int RED_FP_ITEMS = 2;
 
 // The CTA has TT compute threads (one 128-byte row each) plus one look-back
 // warp.  The look-back warp issues the tile's TMA load and at once starts
@@ -592,8 +599,8 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
   // whose segment began before these items, waits for the earlier threads'
   // prefix (first_s, first_v).  Float64 + over longer segments (FOLD) does so
   // only in warps where a segment starts or ends; the others (their rows are
-  // full, or all past the end) fold theirs in fixed point, all 16 items (the
-  // last two in FP64 as well: 95 us against 90 at 1100 elements a segment).
+  // full, or all past the end) fold theirs in fixed point but for the last
+  // RED_FP_ITEMS items.
   constexpr bool FOLD = MODE == M_REDUCE && std::is_same<Op, AddD>::value && !CHAIN;
   int first_s = -1;
   T first_v = Op::ident();
@@ -604,7 +611,14 @@ __global__ void __launch_bounds__(cta_threads<MODE>(), tma_minb<MODE, typename O
     folded = !__any_sync(0xffffffffu, heads != 0 || nh);
     if (folded) {
       tf = 0;
-      tv = cnt > 0 ? fx_range<ITEMS>(x, 0, ITEMS) : AddD::ident();
+      tv = AddD::ident();
+      if (cnt > 0) {
+        constexpr int H = ITEMS - RED_FP_ITEMS;
+        double hi = x[H];
+#pragma unroll
+        for (int i = H + 1; i < ITEMS; i++) hi = __dadd_rn(hi, x[i]);
+        tv = __dadd_rn(fx_range_part<ITEMS, 0, H>(x, 0, ITEMS), hi);
+      }
     }
   }
   if (SEG && MODE == M_REDUCE && !folded) {

@@ -352,3 +352,14 @@ def test_descriptors_of_mostly_empty_segments(gpu, oracle, n, m, where):
         R.got = [ops.scan_e(R, "add_sez", x, lens), ops.reduce_e(R, "max_rez", x, lens), ops.dis_e(R, "dis_vez", v, lens)]
     for a, b in zip(gpu.got, oracle.got):
         assert np.array_equal(a, b)
+
+
+def test_float_sums_keep_the_small_items_of_a_row(gpu):
+    """Rows of 16 whose last item is 2^52 times the others: every sum on the way is a float64, so the results are
+    exact unless items are cut off at the unit of a row's largest."""
+    m, per = 3, 8 * 2048  # segments of eight tiles
+    row = np.zeros(16)
+    row[:8], row[15] = 2.0 ** -53, 1.0
+    x = np.tile(row, m * per // 16)
+    got = ops.reduce_e(gpu, "add_red", x, np.full(m, per, dtype=np.int32))
+    assert np.array_equal(got, np.full(m, per // 16 * (1.0 + 2.0 ** -50)))
