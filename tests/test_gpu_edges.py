@@ -1,6 +1,8 @@
 """Kernels at the sizes where a branch of their dispatch or an edge of their
 tiles could go wrong, against the oracle.  Whole numbers and moved values are
 compared bit for bit."""
+import math
+
 import numpy as np
 import pytest
 
@@ -363,3 +365,13 @@ def test_float_sums_keep_the_small_items_of_a_row(gpu):
     x = np.tile(row, m * per // 16)
     got = ops.reduce_e(gpu, "add_red", x, np.full(m, per, dtype=np.int32))
     assert np.array_equal(got, np.full(m, per // 16 * (1.0 + 2.0 ** -50)))
+
+
+@pytest.mark.parametrize("n", [513, 1000, 8191, 8192])
+def test_float_sum_of_a_short_vector_is_folded_pairwise(gpu, n):
+    """One large element in each of the first 512, then ones that a running sum rounds up every time: pairwise,
+    an element takes part in at most 4 + 5 + 4 inexact additions, 2^-53 each."""
+    x = np.full(n, 2.0 ** -53 * (1 + 2.0 ** -7))
+    x[:512] = 1.0
+    exact = math.fsum(x)
+    assert abs(ops.reduce_u(gpu, "add_rud", x) - exact) <= 13 * 2.0 ** -53 * exact
