@@ -564,35 +564,76 @@ template <class T> void lw_fix_seg(T *d, const T *s, const LwMem &L, const int *
 //   2^20   3 n      55 /  58 -> 19/ 22   74/  76 ->  24/ 26   113/ 115 ->  25/ 27
 //   2^22   3 n     109 / 147 -> 44/ 61  187/ 257 ->  67/ 84   300/ 416 ->  66/ 82
 //   2^24   3 n     261 / 390 ->212/271  574/ 791 -> 576/743  1759/2039 -> 563/713
-// The line lies at the last row: beyond it the owners are far larger than L2,
+//   2^25     n     279 ->       162     761 ->      846      2216 ->      741
+//   3*2^24   n     386 ->       239    1095 ->     1668      3744 ->     1448
+// The line lies at the last row of each: beyond it the owners are far larger than L2,
 // and each of unique destinations' atomics is a DRAM read-modify-write of a
 // sector where the form above only sets a bit.
 constexpr long PUT_OWNER_MAX = 3L << 24;
 inline bool put_by_owner(long n_d) { return n_d <= PUT_OWNER_MAX; }
 inline size_t put_bytes(long n_d) { return align_up((size_t)n_d * 4, 256) + 256; }
-__global__ void __launch_bounds__(VBLOCK) k_put_owner(const int *__restrict__ idx, const int *__restrict__ f, long n,
-                                                      long n_d, int *__restrict__ owner) {
+// Few values for many destinations clear the owners of their own destinations
+// alone and store as their owners, so that nothing but the copy of a default
+// that lies apart grows with the destinations.  Where the owners of all are
+// cleared and read, fpm_pu* of 48 values into 3 * 2^24 ints took 79 us, this
+// takes 12, the check-scatter-fix form 27.  That form / owners of all / of the
+// values' destinations, ints, us (asc: ascending, uniq: unique, rep: repeated):
+//   fpm_puz  n_d   n_d/n_s  asc            rep          dpe_puz  n_d  n_d/n_s  uniq
+//           2^23    32      33/ 25/ 21     41/ 25/ 21           2^25   32    159/113/157
+//           2^25    16      66/100/ 90    193/106/117           2^25  128    119/ 91/ 79
+//           2^25    32      52/ 91/ 69    119/ 87/ 62         3*2^24  128    148/137/114
+//           2^25   128      35/ 70/ 21     68/ 71/ 21
+//         3*2^24    32      68/137/110    176/131/104
+// Between 4 and 48 destinations per value from 2^25 of them on the form that
+// checks is the fastest for ascending and unique ones and the slowest for
+// repeated ones; the owner forms lie between, and the line where they meet.
+inline bool put_sparse(long n_s, long n_d, bool copied) {
+  return copied ? n_d >= 1L << 25 && n_s <= n_d / 128 : n_d >= 1L << 23 && n_s <= n_d / 32;
+}
+// What a pass over the elements does with one whose destination is g: clear
+// its owner, become its owner, or store as its owner.
+enum { PUT_CLEAR, PUT_OWN, PUT_STORE };
+template <int STEP, class T>
+__global__ void __launch_bounds__(VBLOCK) k_put_walk(const int *__restrict__ idx, const int *__restrict__ f, long n,
+                                                     long n_d, int *__restrict__ owner, T *__restrict__ d,
+                                                     const T *__restrict__ s) {
   const long i0 = (long)blockIdx.x * (VBLOCK * GITEMS) + threadIdx.x;
   int g[GITEMS];
+  T x[STEP == PUT_STORE ? GITEMS : 1];
   bool ok[GITEMS];
 #pragma unroll
   for (int u = 0; u < GITEMS; u++) {
     const long k = i0 + (long)u * VBLOCK;
     ok[u] = k < n;
     g[u] = ok[u] ? __ldcs(idx + k) : -1;
+    if constexpr (STEP == PUT_STORE)
+      if (ok[u]) x[u] = __ldcs(s + k);
     if (f && ok[u]) ok[u] = __ldcs(f + k) != 0;
+  }
+  if constexpr (STEP == PUT_STORE) {
+#pragma unroll
+    for (int u = 0; u < GITEMS; u++)
+      ok[u] = ok[u] && g[u] >= 0 && g[u] < n_d && owner[g[u]] == (int)(i0 + (long)u * VBLOCK);
   }
 #pragma unroll
   for (int u = 0; u < GITEMS; u++)
-    if (ok[u] && g[u] >= 0 && g[u] < n_d) atomicMax(owner + g[u], (int)(i0 + (long)u * VBLOCK));
+    if (ok[u] && g[u] >= 0 && g[u] < n_d) {
+      if constexpr (STEP == PUT_CLEAR) owner[g[u]] = -1;
+      else if constexpr (STEP == PUT_OWN) atomicMax(owner + g[u], (int)(i0 + (long)u * VBLOCK));
+      else d[g[u]] = x[u];
+    }
 }
 // the segmented forms: the destination of k is off_d[segment of k] + i[k]
-struct PutOwnerSeg {
-  const int *i; const int *f; const int *off_d; int m_d; long n_d; int *owner;
+template <int STEP, class T> struct PutSeg {
+  const int *i; const int *f; const int *off_d; int m_d; long n_d; int *owner; T *d; const T *s;
   __device__ void operator()(int k, int sg, int) const {
     if (sg < m_d && (f == nullptr || __ldg(f + k))) {
       const long g = (long)__ldg(off_d + sg) + __ldg(i + k);
-      if (g >= 0 && g < n_d) atomicMax(owner + g, k);
+      if (g >= 0 && g < n_d) {
+        if constexpr (STEP == PUT_CLEAR) owner[g] = -1;
+        else if constexpr (STEP == PUT_OWN) atomicMax(owner + g, k);
+        else if (owner[g] == k) d[g] = __ldcs(s + k);
+      }
     }
   }
 };
@@ -622,7 +663,17 @@ __global__ void __launch_bounds__(VBLOCK) k_put_take(T *d, const T *__restrict__
 inline int put_units(long n_s, long n_d, bool seg) {
   return (int)(((put_by_owner(n_d) ? put_bytes(n_d) : lw_bytes(n_s, n_d, seg)) + 7) / 8);
 }
-// unsegmented when ss is null
+// one pass over the elements; unsegmented when ss is null
+template <int STEP, class T>
+void put_walk(const int *i, const int *f, long n_s, long n_d, const SegView *ss, const SegView *sdd, int *owner, T *d,
+              const T *s, const char *name) {
+  if (ss) {
+    segwalk(PutSeg<STEP, T>{i, f, sdd->off, sdd->m, n_d, owner, d, s}, *ss, name);
+  } else {
+    k_put_walk<STEP, T><<<grid_for(n_s, VBLOCK * GITEMS), VBLOCK, 0, stream()>>>(i, f, n_s, n_d, owner, d, s);
+    launch_check(name);
+  }
+}
 template <class T>
 void put(T *d, const T *s, const int *i, const int *f, const T *v, int n_s, int n_d, const SegView *ss,
          const SegView *sdd, vec_p scratch, const char *name) {
@@ -630,14 +681,17 @@ void put(T *d, const T *s, const int *i, const int *f, const T *v, int n_s, int 
   void *mem = scratch_or_work(scratch, put_bytes(n_d));
   if (!mem) return;
   int *owner = (int *)align_up((size_t)mem, 256);
-  if (!GCVL_CK(cudaMemsetAsync(owner, 0xFF, (size_t)n_d * 4, stream()))) return;
-  if (ss) {
-    segwalk(PutOwnerSeg{i, f, sdd->off, sdd->m, n_d, owner}, *ss, name);
-  } else {
-    k_put_owner<<<grid_for(n_s, VBLOCK * GITEMS), VBLOCK, 0, stream()>>>(i, f, n_s, n_d, owner);
-    launch_check(name);
+  if (v == d) v = nullptr;
+  if (put_sparse(n_s, n_d, v != nullptr)) {
+    if (v && !GCVL_CK(cudaMemcpyAsync(d, v, (size_t)n_d * sizeof(T), cudaMemcpyDeviceToDevice, stream()))) return;
+    put_walk<PUT_CLEAR, int>(i, f, n_s, n_d, ss, sdd, owner, nullptr, nullptr, name);
+    put_walk<PUT_OWN, int>(i, f, n_s, n_d, ss, sdd, owner, nullptr, nullptr, name);
+    put_walk<PUT_STORE, T>(i, f, n_s, n_d, ss, sdd, owner, d, s, name);
+    return;
   }
-  k_put_take<T><<<grid_for(n_d, VBLOCK * GITEMS), VBLOCK, 0, stream()>>>(d, s, v == d ? nullptr : v, owner, n_d);
+  if (!GCVL_CK(cudaMemsetAsync(owner, 0xFF, (size_t)n_d * 4, stream()))) return;
+  put_walk<PUT_OWN, int>(i, f, n_s, n_d, ss, sdd, owner, nullptr, nullptr, name);
+  k_put_take<T><<<grid_for(n_d, VBLOCK * GITEMS), VBLOCK, 0, stream()>>>(d, s, v, owner, n_d);
   launch_check(name);
 }
 

@@ -375,3 +375,58 @@ def test_float_sum_of_a_short_vector_is_folded_pairwise(gpu, n):
     x[:512] = 1.0
     exact = math.fsum(x)
     assert abs(ops.reduce_u(gpu, "add_rud", x) - exact) <= 13 * 2.0 ** -53 * exact
+
+
+def _dpe_in_place(R, name, x, idx, v, lens=None):
+    """dpe_* whose destination is its own default, as the interpreter issues it when the default dies there."""
+    t = name[-1]
+    d, s, i = R.vec(v, t), R.vec(x, t), R.vec(idx, "z")
+    if lens is None:
+        sizes = a = (len(x), len(v))
+    else:
+        (sds, n_s, m_s), (sdd, n_d, m_d) = R.segd(lens[0]), R.segd(lens[1])
+        sizes, a = (n_s, m_s, n_d, m_d), (R.p(sds), n_s, m_s, R.p(sdd), n_d, m_d)
+    scr = R.units(R.fn(name + "_scratch")(*sizes))
+    R.fn(name)(R.p(d), R.p(s), R.p(i), R.p(d), *a, R.p(scr))
+    r = R.get(d, len(v))
+    R.done()
+    return r
+
+
+# few values for many destinations: from 2^23 destinations and 32 of them per value on, 2^25 and 128 where the
+# default is copied; owners left from other puts lie in the scratch
+@pytest.mark.parametrize("n_d,n_s", [((1 << 23) - 1, 40), (1 << 23, 1), (1 << 23, 40), (1 << 23, 1 << 18), (1 << 23, (1 << 18) + 1),
+                                     ((1 << 25) - 1, 1000), (1 << 25, 2049), (1 << 25, 1 << 18), (1 << 25, (1 << 18) + 1)])
+@pytest.mark.parametrize("t", "zd")
+def test_put_of_few_values(gpu, oracle, t, n_d, n_s):
+    r = W.rng(n_d + n_s)
+    v, x = _keys(r, n_d, t, "few"), _keys(r, n_s, t, "uniform")
+    flags = (r.random(n_s) < 0.6).astype(np.int32)
+    for idx in (r.integers(0, n_d, size=n_s), r.integers(n_d - 9, n_d, size=n_s), np.arange(n_s) * (n_d // n_s)):
+        idx = idx.astype(np.int32)
+        want = v.copy()  # the last value stays
+        want[idx] = x
+        keep = v.copy()
+        keep[idx[flags != 0]] = x[flags != 0]
+        assert np.array_equal(ops.dpe_u(gpu, f"dpe_pu{t}", x, idx, v), want)
+        assert np.array_equal(_dpe_in_place(gpu, f"dpe_pu{t}", x, idx, v), want)
+        assert np.array_equal(ops.fpm_u(gpu, f"fpm_pu{t}", x, idx, flags, n_d, v), keep)
+        assert np.array_equal(ops.fpm_u(gpu, f"dfp_pu{t}", x, idx, flags, n_d, v), keep)
+    assert np.array_equal(ops.dpe_u(oracle, f"dpe_pu{t}", x, idx, v), want)
+
+
+@pytest.mark.parametrize("m,ratio", [(3000, 31), (3000, 33), (3000, 130), (1, 130)])
+@pytest.mark.parametrize("t", "zd")
+def test_put_of_few_values_by_segments(gpu, oracle, t, m, ratio):
+    r = W.rng(m + ratio)
+    len_s = r.multinomial((1 << 25) // ratio, np.ones(m) / m).astype(np.int32)
+    len_d = (len_s * ratio + ((1 << 25) % ratio > 0)).astype(np.int32)
+    len_d[-1] += max(0, (1 << 25) - int(len_d.sum()))
+    idx = W.seg_indices(r, len_d, len_s)
+    x, v = _keys(r, int(len_s.sum()), t, "uniform"), _keys(r, int(len_d.sum()), t, "few")
+    flags = (r.random(x.size) < 0.6).astype(np.int32)
+    for R in (gpu, oracle):
+        R.got = [ops.dpe_e(R, f"dpe_pe{t}", x, idx, v, len_s, len_d), _dpe_in_place(R, f"dpe_pe{t}", x, idx, v, (len_s, len_d)),
+                 ops.fpm_e(R, f"fpm_pe{t}", x, idx, flags, len_s, len_d, v)]
+    for a, b in zip(gpu.got, oracle.got):
+        assert np.array_equal(a, b)
