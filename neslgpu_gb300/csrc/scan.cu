@@ -1441,17 +1441,24 @@ template <class T> constexpr size_t tma_smem(int wmax) {
   return 1024 + (size_t)TT * row_items<T>() * sizeof(T) + (size_t)(wmax > 0 ? wpad(wmax) + 1 : 0) * 4;
 }
 
-// Scans of at most this many elements take k_scan, one tile per CTA: while the
-// tiles are few, the ring's two rounds and its load by TMA only add latency.
-// k_scan / ring, us: add_sez 2^14 6.2 / 8.3, 2^18 6.3 / 8.6, 2^20 10.2 / 12.3,
-// 2^22 14.4 / 16.4, 2^23 22.5 / 18.4; add_suz 2^21 15.3 / 17.0, 2^22 22.3 /
-// 20.5; add_sed 2^14 8.9 / 11.4, 2^18 9.2 / 15.4, 2^19 13.3 / 16.4, 2^20 20.5 /
-// 18.7; max_sed 2^18 10.2 / 17.2, 2^21 30.7 / 42.1, 2^22 50.3 / 51.3, 2^24 166 / 156;
-// mul_sed 2^21 28.7 / 34.5, 2^22 47.4 / 43.0.  Float64 + is added in FP64 there,
-// not in fixed point: the error against exact sums is the smaller of the two.
-template <class Op, bool SEG> constexpr long ring_above() {
-  if (std::is_same<Op, AddD>::value) return 1L << 19;
-  return SEG && !std::is_same<Op, MulD>::value ? 1L << 22 : 1L << 21;
+// Short scans take k_scan, one tile per CTA: while the tiles are few, the
+// ring's two rounds and its load by TMA only add latency.  k_scan / ring, us,
+// among other calls:
+//   4 byte, segments of 64: 2^14 7.9 / 8.3, 2^17 8.4 / 9.0, 2^20 13.4 / 12.3, 3 * 2^20 17.2 / 15.3
+//   4 byte, segments of 3:  2^14 9.0 / 8.2, 2^17 9.9 / 9.0, 2^20 13.6 / 12.2, 3 * 2^20 18.0 / 15.2
+//   4 byte, unsegmented:    2^17 7.1 / 8.6, 2^20 12.1 / 13.5, 2^21 and 3 * 2^20 as the ring
+//   max_sed: 2^17 14.8 / 16.3, 2^20 25.5 / 30.8 in segments of 64 (29.7 / 30.0 of 1100), 2^21 0.87 and
+//     1.05 of the ring's time, 3 * 2^20 51.4 / 49.7 (59.0 / 48.7)
+//   max_sud 2^20 0.99, 1.5 * 2^20 1.26 of the ring's time; mul_sud as much; mul_sed 1.5 * 2^20 0.96, 2^21 1.1
+//   add_sed: 2^17 11.8 / 12.8, 2^19 1.0 to 1.2 of the ring's time, 2^20 20.5 / 18.7
+// Float64 + is added in FP64 there, not in fixed point: the error against
+// exact sums is the smaller of the two, so its line lies as far up as the
+// times are about the same.
+template <class Op, bool SEG> inline bool scan_by_tiles(long n, long m) {
+  if (sizeof(typename Op::T) == 4) return SEG ? n <= 3L << 18 && n >= 8 * m : n <= 1L << 21;
+  if (std::is_same<Op, AddD>::value) return n <= 1L << 19;
+  if (std::is_same<Op, MulD>::value) return n <= (SEG ? 3L << 19 : 1L << 20);
+  return n <= (SEG && n < 256 * m ? 1L << 21 : 1L << 20);  // min, max
 }
 // CTAs of a ring scan: as many as are resident at once (0: it does not fit)
 template <class Op, bool SEG> int ring_grid(int tiles) {
@@ -1499,7 +1506,7 @@ bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n
   CUtensorMap tin, tout;
   State &S = st();
   if constexpr (MODE == M_SCAN) {
-    if (n <= ring_above<Op, SEG>()) return false;
+    if (scan_by_tiles<Op, SEG>(n, m)) return false;
     const int tiles = ceil_div(n, (long)RTT * row_items<T>());
     const int grid = ring_grid<Op, SEG>(tiles);
     if (grid > 0) {

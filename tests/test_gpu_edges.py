@@ -430,3 +430,21 @@ def test_put_of_few_values_by_segments(gpu, oracle, t, m, ratio):
                  ops.fpm_e(R, f"fpm_pe{t}", x, idx, flags, len_s, len_d, v)]
     for a, b in zip(gpu.got, oracle.got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("name,n,mean", [("add_sez", 4097, 7), ("add_sez", 4097, 8), ("xor_sez", 20_003, 7), ("min_sez", 20_003, 8),
+                                         ("add_sez", 3 << 18, 8), ("add_sez", (3 << 18) + 1, 8), ("max_sed", 1 << 20, 256),
+                                         ("max_sed", (1 << 20) + 1, 257), ("min_sed", 1 << 21, 255), ("min_sed", (1 << 21) + 1, 255),
+                                         ("mul_sed", 3 << 19, 50), ("mul_sed", (3 << 19) + 1, 50), ("max_sud", 1 << 20, 0),
+                                         ("max_sud", (1 << 20) + 1, 0), ("mul_sud", 1 << 20, 0), ("mul_sud", (1 << 20) + 1, 0)])
+def test_scans_either_side_of_their_lines(gpu, oracle, name, n, mean):
+    """The sizes and mean segment lengths up to which scans take a tile per CTA."""
+    r = W.rng(n + mean)
+    x = _keys(r, n, name[-1], "uniform")
+    if name[:3] == "mul":  # products exact in any order
+        x = np.where(r.random(n) < 0.5, -1.0, 1.0)
+    if name[5] == "u":
+        assert np.array_equal(ops.scan_u(gpu, name, x), ops.scan_u(oracle, name, x))
+    else:
+        lens = np.array([mean] * (n // mean) + [n % mean] * (n % mean > 0), dtype=np.int32)
+        assert np.array_equal(ops.scan_e(gpu, name, x, lens), ops.scan_e(oracle, name, x, lens))
