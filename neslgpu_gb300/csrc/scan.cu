@@ -1116,6 +1116,7 @@ constexpr unsigned WR_CHUNK_BYTES = WR_ELEMS * 4;
 constexpr size_t wr_warp_bytes() { return (size_t)WR_NB * WR_CHUNK_BYTES; }
 constexpr size_t wr_smem() { return 1024 + WR_WARPS * wr_warp_bytes(); }
 constexpr int WR_MAX_CTAS = 8;  // per SM, for the scratch's size
+constexpr int WR_WAVES = 3;     // times as many ranges as fit at once, where they may be uneven
 
 #ifndef GCVL_WR_MINB
 #define GCVL_WR_MINB 6
@@ -1483,18 +1484,21 @@ template <class Op, bool SEG> int ring_grid(int tiles) {
   return (int)(g < tiles ? g : tiles);
 }
 
-// Four-byte elements in segments of at least this many on average reduce by
+// Four-byte elements in segments of at least WR_MEAN on average reduce by
 // warp ranges, shorter ones by tiles, whose offsets window finds the segments
-// of many ends sooner (max_rez at 2^25, warp ranges / tiles, us: mean 3
-// 104 / 103, 5 78 / 86, 8 63 / 82, 16 49 / 78, 31 42 / 70, 1100 38 / 48).
+// of many ends sooner.  Segments of fewer than WR_MEAN_EVEN elements on average
+// may be short ones in one place and long ones in another, and the ranges of
+// the short ones take longest: three times as many ranges as fit at once let
+// the GPU balance them.  max_rez at 2^25, ranges / three times as many / tiles,
+// us: even segments of 5 87 / 87 / 95; geometric of mean 6 68 / 75 / 94, 8 60 /
+// 66 / 91, 10 56 / 61 / 91, 16 49 / 54 / 87, 1100 37 / 41 / 45; half the
+// elements in four segments and the others of mean 2.5 (5 in all) 109 / 96 /
+// 81, 3 (6) 95 / 84 / 76, 4 (8) 82 / 72 / 74, 5 (10) 73 / 70 / 76.
 // Eight-byte elements stay on tiles: in warp ranges each lane's chain of
 // compares or FP64 products is the time (mul_red at mean 64 186 us against
 // 125, max_red 193 against 201), and on the ring scan's rounds with its
 // look-back they took twice as long (302 and 399).
-#ifndef GCVL_WR_MEAN
-#define GCVL_WR_MEAN 5
-#endif
-constexpr long WR_MEAN = GCVL_WR_MEAN;
+constexpr long WR_MEAN = 6, WR_MEAN_EVEN = 9;
 // Returns false (nothing launched) when the vectors do not suit TMA.
 template <class Op, int MODE, bool SEG>
 bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n, int m, vec_p scratch,
@@ -1527,7 +1531,7 @@ bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n
   }
   if constexpr (MODE == M_REDUCE && SEG && sizeof(T) == 4) {
     if ((long)n >= WR_MEAN * m) {
-      // per-warp ranges: as many as fit at once, at most one per chunk
+      // per-warp ranges: as many as fit at once or three times that, at most one per chunk
       const long chunks = ceil_div(n, (long)WR_ELEMS);
       static int per_sm = -1;
       if (per_sm < 0) {
@@ -1537,7 +1541,8 @@ bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n
           GCVL_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_segred_warp<Op>, WR_WARPS * 32,
                                                                 wr_smem()));
       }
-      const long ranges = std::min((long)std::clamp(per_sm, 1, WR_MAX_CTAS) * S.sm_count * WR_WARPS, chunks);
+      const int waves = (long)n < WR_MEAN_EVEN * m ? WR_WAVES : 1;
+      const long ranges = std::min((long)std::clamp(per_sm, 1, WR_MAX_CTAS) * waves * S.sm_count * WR_WARPS, chunks);
       if (!tma_map<T>(&tin, in, rows, 32)) return false;
       void *mem = scratch_or_work(scratch, reduce_pass_bytes((int)ranges));
       if (!mem) return true;
@@ -1828,7 +1833,7 @@ template <class T> int seg_reduce_units(int n) {
   const size_t pass = reduce_pass_bytes(a > b ? a : b);
   if (sizeof(T) == 8) return (int)((pass + 7) / 8);
   const long sms = st().sm_count > 0 ? st().sm_count : 152;  // and the warp ranges'
-  const long ranges = std::min(sms * WR_MAX_CTAS * WR_WARPS, (long)ceil_div(n, (long)WR_ELEMS));
+  const long ranges = std::min(sms * WR_MAX_CTAS * WR_WAVES * WR_WARPS, (long)ceil_div(n, (long)WR_ELEMS));
   return (int)((std::max(pass, reduce_pass_bytes((int)ranges)) + 7) / 8);
 }
 template <class T> int reduce_units(int n) {

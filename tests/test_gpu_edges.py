@@ -448,3 +448,25 @@ def test_scans_either_side_of_their_lines(gpu, oracle, name, n, mean):
     else:
         lens = np.array([mean] * (n // mean) + [n % mean] * (n % mean > 0), dtype=np.int32)
         assert np.array_equal(ops.scan_e(gpu, name, x, lens), ops.scan_e(oracle, name, x, lens))
+
+
+@pytest.mark.parametrize("n", [6000, 1 << 20, (1 << 24) + 1025])
+@pytest.mark.parametrize("mean", [5, 6, 8, 9])
+@pytest.mark.parametrize("shape", ["even", "uneven"])
+def test_reductions_either_side_of_the_warp_ranges(gpu, oracle, shape, mean, n):
+    """Warp ranges from 6 elements a segment on, three times as many below 9; short segments and long ones apart."""
+    r = W.rng(n + mean)
+    if shape == "even":
+        lens = np.array([mean] * (n // mean) + [n % mean] * (n % mean > 0), dtype=np.int32)
+    else:  # mean * m elements: m - 2 segments of half the mean among two long ones
+        m = n // mean
+        lens = np.full(m, max(1, mean // 2), dtype=np.int32)
+        lens[m // 5] = lens[m // 2] = 0
+        lens[m // 5] = (n - int(lens.sum())) // 2
+        lens[m // 2] = n - int(lens.sum())
+    x, b = W.int32_uniform(r, n), (r.random(n) < 0.4).astype(np.int32)
+    for R in (gpu, oracle):
+        R.got = [ops.reduce_e(R, "max_rez", x, lens), ops.reduce_e(R, "add_rez", x, lens), ops.pk1_e(R, b, lens),
+                 ops.reduce_e(R, "ior_reb", b, lens)]
+    for g, o in zip(gpu.got, oracle.got):
+        assert np.array_equal(g, o)
