@@ -1709,12 +1709,14 @@ static void run_gather_mul_reduce(double *y, const double *vals, const int *cols
 constexpr int RBLOCK = 512;
 // One CTA up to here: it needs no ticket, so nothing is cleared first (1000
 // elements: the clear, 4.6 us and a copy of the result, now 3.1 us).
-// It folds its items pairwise, 16 a thread, then the lanes' and the warps': 13
-// roundings of a sum on the way.  A running fold per thread and over the warps
-// (37 roundings) raised the mean error of float64 sums of 1000 to 8192
-// exponential values from 0.6 to 0.9 units in the last place.
-constexpr int RED_ALONE_ITEMS = 16;
-constexpr long RED_ALONE_MAX = RBLOCK * RED_ALONE_ITEMS;
+// It folds the 16 warps' results pairwise: one after another, the largest sums
+// take the most roundings, and the mean error of float64 sums of 1000 to 8192
+// exponential values was 0.7 to 0.9 units in the last place, now 0.6.  (Folding
+// a thread's up to 16 items pairwise as well changes no digit of that, and its
+// unrolled code takes 2 us more, 8.3 against 6.2 at 1000 elements.)
+// One CTA / several, us: add_red in one segment 4096 6.2 / 8.0, 8192 9.3 / 8.2,
+// max_red 4096 8.3 / 10.2, 6000 10.3 / 10.3; add_rez 8192 4.1 / 6.2.
+template <class T> constexpr long red_alone_max() { return sizeof(T) == 8 ? 4096 : 8192; }
 template <class Op>
 __global__ void __launch_bounds__(RBLOCK) k_reduce(const typename Op::T *__restrict__ in, long n,
                                                   typename Op::T *partial, unsigned *ticket,
@@ -1728,26 +1730,11 @@ __global__ void __launch_bounds__(RBLOCK) k_reduce(const typename Op::T *__restr
   long per = (n + gridDim.x - 1) / gridDim.x;
   long lo = (long)blockIdx.x * per, hi = min(n, lo + per);
   (void)stride;
-  auto item = [&](long i) {
-    const T x = __ldcs(in + i);
-    return count_flags ? (x != (T)0 ? (T)1 : (T)0) : x;
-  };
-  const bool alone = gridDim.x == 1;
-  if (alone) {
-    T v[RED_ALONE_ITEMS];
-#pragma unroll
-    for (int q = 0; q < RED_ALONE_ITEMS; q++) {
-      const long i = threadIdx.x + q * RBLOCK;
-      v[q] = i < n ? item(i) : Op::ident();
-    }
-#pragma unroll
-    for (int h = RED_ALONE_ITEMS / 2; h > 0; h /= 2)
-#pragma unroll
-      for (int q = 0; q < h; q++) v[q] = Op::apply(v[q], v[q + h]);
-    acc = v[0];
-  } else {
 #pragma unroll 8
-    for (long i = lo + threadIdx.x; i < hi; i += RBLOCK) acc = Op::apply(acc, item(i));
+  for (long i = lo + threadIdx.x; i < hi; i += RBLOCK) {
+    T x = __ldcs(in + i);
+    if (count_flags) x = (x != (T)0) ? (T)1 : (T)0;
+    acc = Op::apply(acc, x);
   }
   // thread order within a warp, then warps in order
 #pragma unroll
@@ -1757,7 +1744,7 @@ __global__ void __launch_bounds__(RBLOCK) k_reduce(const typename Op::T *__restr
   }
   if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = acc;
   __syncthreads();
-  if (alone) {  // the only CTA: the result at once, no ticket
+  if (gridDim.x == 1) {  // the only CTA: the result at once, no ticket
     if (threadIdx.x < 32) {
       T b = threadIdx.x < RBLOCK / 32 ? s_w[threadIdx.x] : Op::ident();
 #pragma unroll
@@ -1812,7 +1799,7 @@ void run_reduce(const typename Op::T *in, int n, typename Op::T *result_dev, vec
   int grid = S.sm_count * 2;
   long need = ((long)n + RBLOCK - 1) / RBLOCK;
   if (grid > need) grid = (int)need;
-  if (n <= RED_ALONE_MAX) grid = 1;
+  if (n <= red_alone_max<T>()) grid = 1;
   unsigned *ticket = nullptr;
   T *partial = nullptr;
   if (grid > 1) {

@@ -367,14 +367,14 @@ def test_float_sums_keep_the_small_items_of_a_row(gpu):
     assert np.array_equal(got, np.full(m, per // 16 * (1.0 + 2.0 ** -50)))
 
 
-@pytest.mark.parametrize("n", [513, 1000, 8191, 8192])
-def test_float_sum_of_a_short_vector_is_folded_pairwise(gpu, n):
-    """One large element in each of the first 512, then ones that a running sum rounds up every time: pairwise,
-    an element takes part in at most 4 + 5 + 4 inexact additions, 2^-53 each."""
-    x = np.full(n, 2.0 ** -53 * (1 + 2.0 ** -7))
-    x[:512] = 1.0
+@pytest.mark.parametrize("n", [500, 512])
+def test_float_sum_of_a_short_vector_folds_its_warps_pairwise(gpu, n):
+    """The first warp's 32 elements sum to 1, each other warp's to what a running sum rounds up every time: pairwise,
+    an element takes part in at most 5 + 4 inexact additions, 2^-53 each."""
+    x = np.full(n, 2.0 ** -58 * (1 + 2.0 ** -7))
+    x[:32] = 2.0 ** -5
     exact = math.fsum(x)
-    assert abs(ops.reduce_u(gpu, "add_rud", x) - exact) <= 13 * 2.0 ** -53 * exact
+    assert abs(ops.reduce_u(gpu, "add_rud", x) - exact) <= 9 * 2.0 ** -53 * exact
 
 
 def _dpe_in_place(R, name, x, idx, v, lens=None):
@@ -470,3 +470,10 @@ def test_reductions_either_side_of_the_warp_ranges(gpu, oracle, shape, mean, n):
                  ops.reduce_e(R, "ior_reb", b, lens)]
     for g, o in zip(gpu.got, oracle.got):
         assert np.array_equal(g, o)
+
+
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 8191, 8192, 8193])
+def test_float_reductions_by_one_cta_or_several(gpu, oracle, n):
+    x = W.rng(n).integers(-9, 10, size=n).astype(np.float64)  # sums exact in any order
+    for name in ("add_rud", "max_rud", "min_rud"):
+        assert ops.reduce_u(gpu, name, x) == ops.reduce_u(oracle, name, x)
