@@ -907,6 +907,14 @@ inline int sc_grid(long n) {
   return (int)(need < cap ? (need < 1 ? 1 : need) : cap);
 }
 inline size_t rk_state_bytes(long n) { return (size_t)ceil_div(n, rk_tile(n)) * 256 * 4; }
+// of any vector of at most n elements (a shorter one in smaller tiles may have
+// more of them), so that scratch of a call covers every shorter call
+inline size_t rk_state_room(long n) {
+  size_t b = rk_state_bytes(n);
+  for (const long line : {(long)RK_TINY_MAX, (long)RK_SMALL_MAX})
+    if (n > line) b = std::max(b, rk_state_bytes(line));
+  return b;
+}
 inline int ws_tiles(long n) { return (int)((n + WS_TILE - 1) / WS_TILE); }  // tiles of the window split
 // top-8-bit windows of [0, n)
 inline int window_shift(int n) { int b = bit_length((unsigned)(n > 1 ? n - 1 : 1)); return b > 8 ? b - 8 : 0; }
@@ -1126,7 +1134,7 @@ inline RankLayout rank_layout(int n, int is_double, int seg) {
   L.hist = take(RK_MAXPASS * 256 * 4);  // these three are cleared together
   L.counter = take((RK_MAXPASS + 2) * 4);  // tickets, the long segments' meetings, and whether a wait gave up
   L.lsum = take(8);
-  L.state = take(rk_state_bytes(n) * 3);
+  L.state = take(rk_state_room(n) * 3);
   L.key_a = take((size_t)n * ks);
   L.key_b = take((size_t)n * ks);
   L.idx_a = take((size_t)n * 4);

@@ -77,3 +77,22 @@ def test_scratch_covers_the_kernels_tiles():
             red = _lookback_bytes(t) + -(-t * 4 // 256) * 256 + _lookback_bytes(-(-t // 1024))
             assert 8 * c.add_red_scratch(n, m) >= red, (n, m)
             assert 8 * c.gcvl_spmv_csr_scratch(n, m) >= red, (n, m)
+
+
+def test_scratch_of_a_call_covers_every_shorter_call():
+    """A program may keep one scratch vector, sized for its longest vectors: no F_scratch falls as a size grows
+    (checked around powers of two and three times them, where the forms of a call change)."""
+    from neslgpu_gb300 import abi
+    from neslgpu_gb300.cvl import load
+    c = load()
+    sizes = sorted({k * (1 << e) + d for e in range(27) for k in (1, 3) for d in (-1, 0, 1)} - {0, -1})
+    sizes = [n for n in sizes if n <= 3 << 25]
+    shapes = {1: [lambda n: (n,)], 2: [lambda n: (n, n), lambda n: (n, -(-n // 50)), lambda n: (1 << 26, n + 1)],
+              4: [lambda n: (n, n, n, n), lambda n: (n, 2, 1 << 26, 2), lambda n: (1 << 20, 2, n, 2)]}
+    falls = []
+    for name in abi.CVL:
+        f = getattr(c, name + "_scratch", None)
+        for shape in shapes.get(len(f.argtypes), []) if f else []:
+            units = [f(*shape(n)) for n in sizes]
+            falls += [(name, shape(a), shape(b)) for a, b, ua, ub in zip(sizes, sizes[1:], units, units[1:]) if ub < ua]
+    assert not falls, falls[:5]
