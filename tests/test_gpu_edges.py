@@ -477,3 +477,48 @@ def test_float_reductions_by_one_cta_or_several(gpu, oracle, n):
     x = W.rng(n).integers(-9, 10, size=n).astype(np.float64)  # sums exact in any order
     for name in ("add_rud", "max_rud", "min_rud"):
         assert ops.reduce_u(gpu, name, x) == ops.reduce_u(oracle, name, x)
+
+
+@pytest.mark.parametrize("lens", [(127,), (128,), (129,), (100, 155), (100, 156), (100, 157), (5, 1111, 0, 3000)])
+@pytest.mark.parametrize("form", ["add_red", "spmv"])
+def test_float_sums_either_side_of_the_fold(gpu, oracle, form, lens):
+    """The mean of 128 elements a segment from which warps without a segment boundary fold theirs in fixed point, for
+    sums and for the fused row sums of a sparse matrix; the last has warps with and without a boundary in one tile."""
+    r = W.rng(sum(lens))
+    lens = np.array(lens * (600_000 // sum(lens)), dtype=np.int32)
+    n, m = int(lens.sum()), lens.size
+    x = W.float64_normal(r, n) * 2.0 ** r.integers(-40, 40, size=n)
+    if form == "add_red":
+        g = ops.reduce_e(gpu, "add_red", x, lens)
+    else:
+        c = gpu.cvl
+        w = W.float64_normal(r, 5000)
+        cols = r.integers(0, w.size, size=n).astype(np.int32)
+        sd, _, _ = gpu.segd(lens)
+        vv, cv, wv, y = gpu.vec(x, "d"), gpu.vec(cols, "z"), gpu.vec(w, "d"), gpu.out(m, "d")
+        scr = gpu.units(c.gcvl_spmv_csr_scratch(n, m))
+        c.gcvl_spmv_csr(y.ptr, vv.ptr, cv.ptr, wv.ptr, sd.ptr, n, m, scr.ptr)
+        g = gpu.get(y, m)
+        assert c.gcvl_sync() == 0
+        x = x * w[cols]
+    o = ops.reduce_e(oracle, "add_red", x, lens)
+    e = np.cumsum(lens.astype(np.int64))
+    mag = np.where(lens > 0, np.add.reduceat(np.append(np.abs(x), 0.0), np.minimum(e - lens, n - 1)), 0.0)
+    assert np.all(np.abs(g - o) <= 1e-12 * mag)
+
+
+@pytest.mark.parametrize("shape", ["ones", "limit", "empties", "whole", "vector"])
+@pytest.mark.parametrize("name", ["rku", "rkd"])
+def test_ranks_with_nans(gpu, oracle, name, shape):
+    """NaNs rank by their bits, beyond the infinities of their sign; the buckets of a local rank put them at the ends."""
+    r = W.rng(len(shape))
+    lens = np.array([4000], dtype=np.int32) if shape == "vector" else _segments(r, shape)
+    x = _keys(r, int(lens.sum()), "d", "special")
+    nan = r.random(x.size) < 0.2
+    bits = r.integers(1, 1 << 52, size=x.size, dtype=np.uint64) | np.uint64(0x7FF << 52)
+    bits[r.random(x.size) < 0.5] |= np.uint64(1 << 63)
+    x[nan] = bits.view(np.float64)[nan]
+    if shape == "vector":
+        assert np.array_equal(ops.rank_u(gpu, name + "_lud", x), ops.rank_u(oracle, name + "_lud", x))
+    else:
+        assert np.array_equal(ops.rank_e(gpu, name + "_led", x, lens), ops.rank_e(oracle, name + "_led", x, lens))
