@@ -605,7 +605,7 @@ class Interpreter:
             self.ops_run += 1
             if op == "COPY":
                 k, d = ins.a, ins.b
-                if k == 1:
+                if k == 1 and d < len(st):
                     v = st[-1 - d]
                     v.ref += 1
                     st.append(v)
@@ -616,7 +616,7 @@ class Interpreter:
                 st.extend(seg)
             elif op == "CPOP":
                 k, d = ins.a, ins.b
-                if k == 1:
+                if k == 1 and d < len(st):
                     st.append(st.pop(-1 - d))
                     continue
                 lo, hi = len(st) - d - k, len(st) - d
@@ -625,7 +625,7 @@ class Interpreter:
                 st.extend(seg)
             elif op == "POP":
                 k, d = ins.a, ins.b
-                if k == 1:
+                if k == 1 and d < len(st):
                     self.drop(st.pop(-1 - d))
                     continue
                 lo, hi = len(st) - d - k, len(st) - d
@@ -692,7 +692,7 @@ class Interpreter:
             self.ops_run += 1
             if op == "COPY":
                 k, d = ins.a, ins.b
-                if k == 1:
+                if k == 1 and d < len(st):
                     v = st[-1 - d]
                     v.ref += 1
                     st.append(v)
@@ -703,7 +703,7 @@ class Interpreter:
                 st.extend(seg)
             elif op == "CPOP":
                 k, d = ins.a, ins.b
-                if k == 1:
+                if k == 1 and d < len(st):
                     st.append(st.pop(-1 - d))
                     continue
                 lo, hi = len(st) - d - k, len(st) - d
@@ -712,7 +712,7 @@ class Interpreter:
                 st.extend(seg)
             elif op == "POP":
                 k, d = ins.a, ins.b
-                if k == 1:
+                if k == 1 and d < len(st):
                     self.drop(st.pop(-1 - d))
                     continue
                 lo, hi = len(st) - d - k, len(st) - d

@@ -159,3 +159,12 @@ def test_fused_spmv_matches_vcode_program(gpu, oracle, case, offset):
     want = row_sums(prod) if case == "many" else _spmv(oracle.cvl, lens, cols, vals, x)
     assert np.all(np.abs(got - want) <= 1e-12 * np.maximum(np.abs(want), S) + 1e-300)
     assert np.all(got[lens == 0] == 0.0)
+
+
+@pytest.mark.parametrize("ops,left", [(["POP 1 0"], 0), (["COPY 1 0"], 0), (["CPOP 1 0"], 0), (["CONST INT 3", "COPY 1 1"], 1),
+                                      (["CONST INT 3", "CONST INT 4", "POP 1 2"], 2),
+                                      (["CONST INT 3", "CONST INT 4", "CPOP 1 0"], 2), (["CONST INT 3", "COPY 1 0"], 2)])
+def test_stack_ops_of_one_value_beyond_the_stack(oracle, ops, left):
+    """COPY, POP and CPOP of one value take what the forms for several take: a depth with nothing there moves nothing."""
+    it = V.Interpreter("\n".join(["FUNC MAIN", *ops, "RET"]), oracle.cvl)
+    assert len(it.run("MAIN", [])) == left
