@@ -1190,7 +1190,6 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
     ls.base = (int *)(mem + L.base);
     ls.of_tile = (int *)(mem + L.of_tile);
     rank_local<K>(s, (int *)d, sv, n, up, false, ls);
-    if (n <= LR_MAX) return;  // no segment can be longer
     // the long segments, if there are any: the kernels below return at once otherwise
     total = ls.total;
     const int seg_passes = std::max(1, (bit_length((unsigned)(n / (LR_MAX + 1) - 1)) + 7) / 8);

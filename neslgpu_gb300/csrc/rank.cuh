@@ -13,13 +13,7 @@ __device__ __forceinline__ unsigned rk_key(unsigned x, int up) { return x ^ (up 
 
 // The tile of a local rank's CTA: the segments that start in LR_T elements,
 // each of at most LR_MAX, so at most LR_CAP elements.
-#ifndef GCVL_LR_T
-#define GCVL_LR_T 2048
-#endif
-#ifndef GCVL_LR_MAX
-#define GCVL_LR_MAX 2048
-#endif
-constexpr int LR_BLOCK = 512, LR_T = GCVL_LR_T, LR_MAX = GCVL_LR_MAX, LR_CAP = LR_T + LR_MAX;
+constexpr int LR_BLOCK = 512, LR_T = 2048, LR_MAX = 2048, LR_CAP = LR_T + LR_MAX;
 inline int lr_tiles(long n) { return (int)((n + LR_T - 1) / LR_T); }
 
 // Segments too long for one CTA, numbered in the order they were met and

@@ -9,8 +9,8 @@
 // from earlier tiles comes from a decoupled look-back over 16-byte status
 // words (a tile that holds a segment head publishes its inclusive value at
 // once; the warp-wide look-back walks 32 tiles per round trip).  Kernels:
-//  * k_scan_ring -- scans of 16-byte aligned vectors: persistent CTAs take
-//    tiles from a ticket counter, move them by TMA through a two-slot ring,
+//  * k_scan_ring -- long scans of 16-byte aligned vectors (scan_by_tiles has
+//    the line): persistent CTAs take tiles from a ticket counter, move them by TMA through a two-slot ring,
 //    and write each tile's outputs one round after its fold, so the carry
 //    it needs is ready;
 //  * k_segred_warp -- segmented reductions of 4-byte elements with segments
@@ -20,8 +20,9 @@
 //    tile per CTA, results at segment ends and no look-back wait:
 //    k_tile_fix completes the results that span tiles or warp ranges (and
 //    the no-alloc scan);
-//  * k_scan -- everything else (vectors off a 16-byte boundary, the offsets
-//    scan of mke_fov), staged with coalesced loads.
+//  * k_scan -- everything else (short scans, vectors of one tile, vectors off
+//    a 16-byte boundary, the offsets scan of mke_fov), staged with coalesced
+//    loads, a tile per CTA.
 // Every wait is bounded.
 #include "gcvl.cuh"
 #include "tma.cuh"
