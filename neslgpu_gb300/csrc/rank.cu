@@ -1192,7 +1192,8 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
     rank_local<K>(s, (int *)d, sv, n, up, false, ls);
     // the long segments, if there are any: the kernels below return at once otherwise
     total = ls.total;
-    const int seg_passes = std::max(1, (bit_length((unsigned)(n / (LR_MAX + 1) - 1)) + 7) / 8);
+    // the numbers of as many long segments as there can be
+    const int seg_passes = std::max(1, (bit_length((unsigned)(std::min(m, n / (LR_MAX + 1)) - 1)) + 7) / 8);
     const int pg = std::min(S.sm_count * 8, lr_tiles(n));
     k_rank_prep_long<K><<<pg, RK_BLOCK, 0, S.stream>>>((const K *)s, n, up, sv, ls, seg_passes, (K *)kA, iA, aA, hist,
                                                        state[0], (long)(state_bytes / 4), rk_tile(n));

@@ -522,3 +522,14 @@ def test_ranks_with_nans(gpu, oracle, name, shape):
         assert np.array_equal(ops.rank_u(gpu, name + "_lud", x), ops.rank_u(oracle, name + "_lud", x))
     else:
         assert np.array_equal(ops.rank_e(gpu, name + "_led", x, lens), ops.rank_e(oracle, name + "_led", x, lens))
+
+
+@pytest.mark.parametrize("m", [2, 255, 256, 257, 1000])
+@pytest.mark.parametrize("name", ["rku_lez", "rkd_led"])
+def test_ranks_of_few_long_segments(gpu, oracle, name, m):
+    """The passes by segment number cover as many long segments as there are segments, not as many as would fit."""
+    r = W.rng(m)
+    lens = r.integers(2049, 30_000, size=m).astype(np.int32)
+    lens[m // 2] = 600_000
+    x = _keys(r, int(lens.sum()), name[-1], "few")
+    assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
