@@ -46,8 +46,11 @@ namespace gcvl {
 
 // Keys per thread of a digit pass (tile = 256 x RK_ITEMS), and the CTAs per
 // SM of the 32-bit unsegmented passes, measured at 2^28 (int / double /
-// segmented int rank): 16 items at 4 CTAs 9.09 / 21.4 / 18.0 ms; 20 at 3
-// 9.06 / 19.8 / 17.2; 24 at 3 9.43 / 18.7 / 17.0; 32 at 2 10.1 / 25.9 / 21.9.
+// segmented int rank, every pass over all elements): 16 items at 4 CTAs 9.09 /
+// 21.4 / 18.0 ms; 20 at 3 9.06 / 19.8 / 17.2; 24 at 3 9.43 / 18.7 / 17.0; 32 at
+// 2 10.1 / 25.9 / 21.9.  Now 8.39 / 19.5 ms; segmented, int / double, by log-normal
+// lengths 14.9 / 25.0 (17.8 / 29.0 then), in segments of 20000, all of them
+// long, 17.0 / 30.0 (16.2 / 27.4: there the compaction comes on top).
 #ifndef GCVL_RK_ITEMS
 #define GCVL_RK_ITEMS 20
 #endif
@@ -1084,7 +1087,9 @@ template void scatter_partitioned<unsigned long long>(unsigned long long *, cons
 // grouped by window of the index: window w's pairs lie from slot w << wshift
 // on, as many as the last pass counted (all the window's indices when the
 // vector was ranked whole).  One CTA per 2048 slots, as k_window_scatter;
-// DYN (long segments, usually none): a resident grid.  After a wait of the
+// DYN (long segments, usually none): a resident grid, which takes the slots in
+// ticket order (each CTA striding through them, the CTAs drift apart over the
+// windows: 2^28 ints, all in long segments, 18.2 ms, now 17.0).  After a wait of the
 // passes gave up the pairs may be anything: DYN, whose counts may be missing
 // too, writes nothing, and otherwise an index is looked at before it is
 // followed (10 us of 340 at 2^26 keys; asking the word in every CTA took 20).
@@ -1093,7 +1098,8 @@ __global__ void __launch_bounds__(RK_BLOCK) k_rank_scatter(int *__restrict__ ran
                                                            const unsigned *__restrict__ ppos, int n, int wshift,
                                                            const unsigned long long *total,
                                                            const unsigned *__restrict__ wstate, int tile_elems,
-                                                           const unsigned *gave_up) {
+                                                           const unsigned *gave_up, unsigned *ticket) {
+  __shared__ unsigned s_block;
   const unsigned *counts = nullptr;  // the last tile's inclusive window counts
   if constexpr (DYN) {
     const long t = (long)(unsigned)*(volatile const unsigned long long *)total;
@@ -1101,7 +1107,15 @@ __global__ void __launch_bounds__(RK_BLOCK) k_rank_scatter(int *__restrict__ ran
     if (*(const volatile unsigned *)gave_up) return;
     counts = wstate + (t - 1) / tile_elems * 256;
   }
-  for (long b = blockIdx.x; b * (RK_BLOCK * SC_ITEMS) < n; b += gridDim.x) {
+  for (;;) {
+    long b = blockIdx.x;
+    if constexpr (DYN) {
+      if (threadIdx.x == 0) s_block = atomicAdd(ticket, 1u);
+      __syncthreads();
+      b = s_block;
+      __syncthreads();
+    }
+    if (b * (RK_BLOCK * SC_ITEMS) >= n) return;
     const long i0 = b * (RK_BLOCK * SC_ITEMS) + threadIdx.x;
     unsigned k[SC_ITEMS], v[SC_ITEMS];
     bool ok[SC_ITEMS];
@@ -1132,7 +1146,7 @@ inline RankLayout rank_layout(int n, int is_double, int seg) {
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += align_up(bytes, 256); return at; };
   L.hist = take(RK_MAXPASS * 256 * 4);  // these three are cleared together
-  L.counter = take((RK_MAXPASS + 2) * 4);  // tickets, the long segments' meetings, and whether a wait gave up
+  L.counter = take((RK_MAXPASS + 3) * 4);  // tickets, the long segments' meetings, whether a wait gave up, the scatter's
   L.lsum = take(8);
   L.state = take(rk_state_room(n) * 3);
   L.key_a = take((size_t)n * ks);
@@ -1246,10 +1260,10 @@ void rank_impl(vec_p d, vec_p s, vec_p sd, int n, int m, vec_p scratch, int is_d
   if (!direct) {
     if (seg)
       k_rank_scatter<true><<<sc_grid(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, total, wstate,
-                                                                  rk_tile(n), gave_up);
+                                                                  rk_tile(n), gave_up, counters + RK_MAXPASS + 2);
     else
       k_rank_scatter<false><<<sc_blocks(n), RK_BLOCK, 0, S.stream>>>((int *)d, pidx, ppos, n, wshift, nullptr, nullptr,
-                                                                     rk_tile(n), nullptr);
+                                                                     rk_tile(n), nullptr, nullptr);
     launch_check("k_rank_scatter");
   }
 }
