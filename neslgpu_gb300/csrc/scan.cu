@@ -2097,7 +2097,7 @@ void make_segdes(vec_p sd, vec_p l, int n, int m, vec_p scratch) {
   } else {
     run_scan<AddZ, M_OFFSETS, false>(off, (const int *)l, len, nullptr, m, 1, scratch, false, "mke_fov");
   }
-  if (m >= (few ? SD_SPARSE : 2 * SD_SPARSE) * n)
+  if (n > 0 && m >= (few ? SD_SPARSE : 2 * SD_SPARSE) * n)  // without elements there is no bitmap to write
     k_segdes_sparse<<<ranges * (SD_RANGE / SD_EBLOCK), SD_EBLOCK, 0, S.stream>>>(off, gran, bits, n, m);
   else if (few) k_segdes<false, 512><<<ranges, 512, 0, S.stream>>>(nullptr, nullptr, off, gran, bits, n, m);
   else

@@ -533,3 +533,25 @@ def test_ranks_of_few_long_segments(gpu, oracle, name, m):
     lens[m // 2] = 600_000
     x = _keys(r, int(lens.sum()), name[-1], "few")
     assert np.array_equal(ops.rank_e(gpu, name, x, lens), ops.rank_e(oracle, name, x, lens))
+
+
+@pytest.mark.parametrize("n,m", [(0, 1), (0, 4096), (0, 4097), (0, 100_000), (1, 5000), (8192, 20_000), (8193, 20_000), (8193, 4097),
+                                 (8192 * 304 + 1, 8192 * 304 * 4 + 4), (8192 * 304, 8192 * 304 * 2)])
+def test_descriptors_end_where_their_size_says(gpu, n, m):
+    """Nothing is written past the units that siz_fos gives, nor past the scratch that mke_fov_scratch gives."""
+    c = gpu.cvl
+    lens = np.zeros(m, dtype=np.int32)
+    lens[: min(n, m)] = 1
+    lens[m // 2] += n - int(lens.sum())
+    guard = np.full(4096, 0x5A5A5A5A, dtype=np.int32)
+    room, scr_room = c.siz_fos(n, m), c.mke_fov_scratch(n, m)
+    sd = gpu.vec(np.concatenate([np.zeros(2 * room, dtype=np.int32), guard]), "z")
+    scr = gpu.vec(np.concatenate([np.zeros(2 * scr_room, dtype=np.int32), guard]), "z")
+    lv = gpu.vec(lens, "z")
+    c.mke_fov(sd.ptr, lv.ptr, n, m, scr.ptr)
+    assert np.array_equal(sd.numpy(2 * room + guard.size)[2 * room:], guard)
+    assert np.array_equal(scr.numpy(2 * scr_room + guard.size)[2 * scr_room:], guard)
+    d = gpu.out(m, "z")
+    c.len_fos(d.ptr, sd.ptr, n, m, None)
+    assert np.array_equal(gpu.get(d, m), lens)
+    assert c.gcvl_sync() == 0
