@@ -51,6 +51,7 @@ template <class T> struct ScanArgs {
   const int *gidx;   // gather-multiply form: element k is in[k] * gsrc[gidx[k]]
   const T *gsrc;
   int *lead;         // reductions: per tile, the result lacking the earlier tiles' part (-1: none)
+  bool wait;         // reductions: take the earlier tiles' part by look-back instead
 };
 
 // Coalesced load of a tile into per-thread blocked registers through padded
@@ -206,15 +207,15 @@ k_scan(ScanArgs<typename Op::T> a) {
   pv = ef ? ev : Op::apply(pv, ev);
   pf |= ef;
 
-  // publish and look back (reductions do not wait: the one result per tile
-  // that lacks the earlier tiles' part is completed by k_tile_fix)
+  // publish and look back (reductions do not wait but with a.wait: the one
+  // result per tile that lacks the earlier tiles' part is completed by k_tile_fix)
   if (warp == 0) {
     // thread 0 holds element `base`: its head bit says whether the tile
     // starts a segment (then no carry from earlier tiles is needed)
     const bool first_head = shfl_idx((int)(heads & 1u), 0) != 0;
     if (lane == 0 && !alone) lb_publish(a.lb.word + tile, (tile == 0 || af) ? TS_INC : TS_AGG, to_bits<T>(av));
     T P = Op::ident();
-    if (MODE != M_REDUCE && tile > 0 && !first_head) {
+    if ((MODE != M_REDUCE || a.wait) && tile > 0 && !first_head) {
       P = lookback_prefix<Op>(a.lb.word, tile, a.status, a.spin_limit);
       if (lane == 0 && !af) lb_publish(a.lb.word + tile, TS_INC, to_bits<T>(Op::apply(P, av)));
     }
@@ -251,7 +252,7 @@ k_scan(ScanArgs<typename Op::T> a) {
         run = Op::apply(run, x[i]);
         if (k0 + i + 1 == end) {
           a.out[s] = run;
-          if (!pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
+          if (!a.wait && !pf && !(heads & ((2u << i) - 1u))) a.lead[tile] = s;  // began in an earlier tile
           int s2 = s + 1;
           while (s2 < m && __ldg(a.sv.off + s2 + 1) == end) { a.out[s2] = Op::init(); ++s2; }
           s = s2;
@@ -1500,6 +1501,16 @@ template <class Op, bool SEG> int ring_grid(int tiles) {
 // 125, max_red 193 against 201), and on the ring scan's rounds with its
 // look-back they took twice as long (302 and 399).
 constexpr long WR_MEAN = 6, WR_MEAN_EVEN = 9;
+// Float64 min and max of short vectors take k_scan with its look-back: results
+// are final when it ends, where a tile form's fix-up is one more launch.
+// max_red, look-back / tile form, us: 4096 elements in segments of 8 12.2 /
+// 16.5, of 1100 11.9 / 15.5; 2^16 in 8 14.5 / 17.5; 2^18 in 8 16.5 / 17.5, in
+// 1100 16.7 / 16.5; 2^19 in 8 21.3 / 17.5, in 1100 21.6 / 15.5.
+// Products and sums stay on the tile form, which combines in a fixed order.
+constexpr long RED_WAIT_MAX = 1L << 18;
+template <class Op> inline bool reduce_waits(long n) {
+  return (std::is_same<Op, MinD>::value || std::is_same<Op, MaxD>::value) && n <= RED_WAIT_MAX;
+}
 // Returns false (nothing launched) when the vectors do not suit TMA.
 template <class Op, int MODE, bool SEG>
 bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n, int m, vec_p scratch,
@@ -1562,6 +1573,7 @@ bool run_scan_tma(typename Op::T *out, const typename Op::T *in, vec_p sd, int n
       return true;
     }
   }
+  if (MODE == M_REDUCE && reduce_waits<Op>(n)) return false;
   if (!tma_map<T>(&tin, in, rows)) return false;
   if (MODE == M_SCAN) { if (!tma_map<T>(&tout, out, rows)) return false; }
   else tout = tin;
@@ -1639,11 +1651,12 @@ void run_scan(typename Op::T *out, const typename Op::T *in, typename Op::T *out
     a.lb = lookback_carve(mem, tiles);
     a.lead = (int *)((char *)a.lb.word + align_up((size_t)tiles * 16, 256));
     GCVL_CK(cudaMemsetAsync(mem, 0, lookback_clear_bytes(tiles), S.stream));
-    if (MODE == M_REDUCE) GCVL_CK(cudaMemsetAsync(a.lead, 0xFF, (size_t)tiles * 4, S.stream));
+    a.wait = MODE == M_REDUCE && reduce_waits<Op>(n);
+    if (MODE == M_REDUCE && !a.wait) GCVL_CK(cudaMemsetAsync(a.lead, 0xFF, (size_t)tiles * 4, S.stream));
   }
   k_scan<Op, MODE, SEG><<<tiles, Tiling<T>::BLOCK, 0, S.stream>>>(a);
   launch_check(name);
-  if (MODE == M_REDUCE) launch_tile_fix<Op>(a.lb.word, a.lead, tiles, out);
+  if (MODE == M_REDUCE && !a.wait) launch_tile_fix<Op>(a.lb.word, a.lead, tiles, out);
 }
 
 // Segmented sums of gathered products, y[r] = sum over row r of

@@ -206,3 +206,34 @@ def test_descriptors_whose_waits_run_out(gpu, oracle, n, m):
             c.gcvl_clear_error()
         gpu.fn("max_rez")(y.ptr, xv.ptr, sd.ptr, n, m, rscr.ptr)
         assert np.array_equal(gpu.get(y, m), want)
+
+
+@pytest.mark.gpu
+def test_float_min_max_whose_waits_run_out(gpu, oracle):
+    """With the wait limit forced to 1 the look-back of a short reduction may give up: right or flagged, nothing past
+    the results, and the next call is right."""
+    c = gpu.cvl
+    r = W.rng(9)
+    n = 200_000
+    lens = np.array([n - 40_000, 30_000, 0, 10_000], dtype=np.int32)
+    x = W.float64_normal(r, n)
+    want = ops.reduce_e(oracle, "max_red", x, lens)
+    sd, _, m = gpu.segd(lens)
+    xv, d = gpu.vec(x, "d"), gpu.vec(np.full(m + 512, 7.5), "d")
+    scr = gpu.units(gpu.fn("max_red_scratch")(n, m))
+    old = c.gcvl_get_spin_limit()
+    assert c.gcvl_sync() == 0
+    try:
+        for limit in (1, old):
+            c.gcvl_set_spin_limit(limit)
+            gpu.fn("max_red")(d.ptr, xv.ptr, sd.ptr, n, m, scr.ptr)
+            code = c.gcvl_sync()
+            assert code in ((0, 3) if limit == 1 else (0,))
+            got = d.numpy(m + 512)
+            assert np.all(got[m:] == 7.5)
+            if code == 0:
+                assert np.array_equal(got[:m], want)
+            c.gcvl_clear_error()
+    finally:
+        c.gcvl_set_spin_limit(old)
+        c.gcvl_clear_error()

@@ -555,3 +555,17 @@ def test_descriptors_end_where_their_size_says(gpu, n, m):
     c.len_fos(d.ptr, sd.ptr, n, m, None)
     assert np.array_equal(gpu.get(d, m), lens)
     assert c.gcvl_sync() == 0
+
+
+@pytest.mark.parametrize("n", [2049, 4096, 4097, 100_003, 1 << 18, (1 << 18) + 1])
+@pytest.mark.parametrize("shape", ["one-element", "long", "geometric", "across"])
+@pytest.mark.parametrize("name", ["min_red", "max_red"])
+def test_float_min_max_either_side_of_the_look_back(gpu, oracle, name, shape, n):
+    """Up to 2^18 elements a tile takes the earlier tiles' part of its first result by look-back; vectors on and off a
+    16-byte boundary."""
+    r = W.rng(n + len(shape))
+    lens = np.array([3, 0, n - 5, 0, 2], dtype=np.int32) if shape == "across" else _lens(r, n, shape)
+    x = _keys(r, n, "d", "special")
+    want = ops.reduce_e(oracle, name, x, lens)
+    assert np.array_equal(ops.reduce_e(gpu, name, x, lens), want)
+    assert np.array_equal(ops.reduce_e(ops.DeviceRunner(gpu.cvl, offset=1), name, x, lens), want)
